@@ -105,6 +105,10 @@ struct fi_handle {
     int persist_grid = 0;
     int persist_minb = 2;  // which k_persist build runs (blocks per SM of its register budget)
     size_t persist_smem = 0;
+    bool resident = false;  // the resident kernel runs the segments (fi_resident.cuh)
+    ResArgs rargs{};
+    int resident_grid = 0;
+    size_t resident_smem = 0;
     unsigned long long* d_trace = nullptr;  // phase timeline of the persistent executor
     // plain form
     PlainBufs p{};
@@ -1646,6 +1650,44 @@ static int plan_layouts(fi_handle* h, int K) {
     return setup_persist(h, K);
 }
 
+// Resident kernel: where the row tiles fit one per SM.  Its tile height is the handle's where
+// that gives at most one tile per SM; else the smallest multiple of it that does, if the
+// handle's is even: even heights pair the same rows in the row transforms (with an odd number
+// of rows, if the last tile is one row high as it is with height 2), so the results do not
+// depend on the choice.  Likewise the column tasks take the smallest multiple of the handle's
+// width that leaves one per SM.  FI_PERSIST_RESIDENT=0 keeps k_persist.
+static int setup_resident(fi_handle* h, int K, int nsm) {
+    h->resident = false;
+    const char* e = getenv("FI_PERSIST_RESIDENT");
+    if ((e && e[0] == '0') || h->stage_inputs) return FI_OK;
+    int hr = h->h_rows, Br = h->B_cols;
+    if (cdiv(h->ny, hr) > nsm) {
+        if (hr % 2) return FI_OK;
+        for (hr += h->h_rows; hr <= 16 && (cdiv(h->ny, hr) > nsm || (h->ny % 2 && h->ny % hr != 1)); hr += h->h_rows) {}
+        if (hr > 16 || hr / h->h_rows > RES_MAX_SUB) return FI_OK;
+    }
+    while (cdiv(h->NH, Br) > nsm && Br + h->B_cols <= 16) Br += h->B_cols;
+    ResArgs& r = h->rargs;
+    r.p = h->pargs;
+    r.p.h_rows = hr;
+    r.p.n_rows = cdiv(h->ny, hr);
+    r.p.B_cols = Br;
+    r.p.n_cols = cdiv(h->NH, Br);
+    r.h_sub = h->h_rows;
+    r.n_part = h->n_rows;
+    r.B_sub = h->B_cols;
+    h->resident_grid = std::min(nsm, std::max(r.p.n_rows, r.p.n_cols));
+    cudaFuncAttributes fa{};
+    CK(cudaFuncGetAttributes(&fa, resident_kernel(0, 0, 1)));
+    const size_t budget = h->smem_optin - fa.sharedSizeBytes - 1024;
+    if (!res_layout(h->nx, h->ny, h->Mx, h->My, K, h->plan_x == h->plan_y, hr, Br, r.p.n_cols, h->h_conv, h->B_conv,
+                    h->resident_grid, budget, &r.L))
+        return FI_OK;
+    h->resident_smem = (size_t)r.L.bytes;
+    h->resident = true;
+    return FI_OK;
+}
+
 // Persistent executor set-up: shared-memory layout, grid = resident blocks (at most
 // two per SM), cooperative launch support.  Falls back to the graph executor.
 static int setup_persist(fi_handle* h, int K) {
@@ -1692,7 +1734,7 @@ static int setup_persist(fi_handle* h, int K) {
     }
     h->persist_grid = nsm * std::min(occ, 2);
     h->persist_smem = smem;
-    return FI_OK;
+    return mb ? FI_OK : setup_resident(h, K, nsm);
 }
 
 // Wait bounds of the device waits (fi_debug_set_wait_limit): negative = the default.
@@ -1711,6 +1753,12 @@ static int persist_fn(fi_handle* h, const void** out) {
         sx = seq_code(px.radix, px.npass);
         sy = seq_code(py.radix, py.npass);
     }
+    if (h->resident) {
+        const void* r = resident_kernel(sx, sy, h->rargs.L.all);
+        CK(cudaFuncSetAttribute(r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->resident_smem));
+        *out = r;
+        return FI_OK;
+    }
     const void* f = persist_kernel(sx, sy, h->persist_minb);
     if (f != persist_kernel(0, 0, h->persist_minb))
         CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->persist_smem));
@@ -1725,9 +1773,13 @@ static int run_segment_persist(fi_handle* h) {
     const long long gp = g_grid_polls.load();
     h->pargs.polls = gp >= 0 ? gp : PERSIST_SPIN_LIMIT;
     h->pargs.bar_extra = (unsigned)g_grid_extra.load();
-    void* args[] = {(void*)&h->pargs};
-    CK(cudaLaunchCooperativeKernel(kfn, dim3(h->persist_grid), dim3(ROW_THREADS), args,
-                                   h->persist_smem, h->stream));
+    h->rargs.p.polls = h->pargs.polls;
+    h->rargs.p.bar_extra = h->pargs.bar_extra;
+    h->rargs.p.trace = h->pargs.trace;
+    void* args[] = {h->resident ? (void*)&h->rargs : (void*)&h->pargs};
+    CK(cudaLaunchCooperativeKernel(kfn, dim3(h->resident ? h->resident_grid : h->persist_grid),
+                                   dim3(h->resident ? res_threads(h->rargs.L.all) : ROW_THREADS), args,
+                                   h->resident ? h->resident_smem : h->persist_smem, h->stream));
     unsigned int bar[4];
     CK(cudaMemcpyAsync(bar, h->d_bar, sizeof(bar), cudaMemcpyDeviceToHost, h->stream));
     RET(read_ctl(h));
@@ -2501,7 +2553,7 @@ extern "C" int fi_get_stats(fi_handle* h, fi_stats* st) {
     st->last_gpu_ms = h->last_gpu_ms;
     st->segments = h->segments;
     st->executor = h->cfg.form == FI_FORM_FP32 ? h->executor : -1;
-    st->grid = h->executor == EXEC_PERSIST ? h->persist_grid : 0;
+    st->grid = h->executor != EXEC_PERSIST ? 0 : h->resident ? h->resident_grid : h->persist_grid;
     return FI_OK;
 }
 

@@ -297,8 +297,8 @@ __global__ void __launch_bounds__(RT, 2) k_ens(EnsArgs a) {
                         const int ai = find_member(P, P.nact, t);
                         const int m = P.act[ai], tile = t - P.off[ai];
                         if (C.cm != m) cache_member(a, C, m, 1, tw_smem, nullptr);
-                        ph_cols<ENS_SEQ>(C.m, C.pl, C.m.px.tw32, ws, tile, C.m.B_cols, C.m.S[stage == 3 ? 1 : 0],
-                                C.m.cpart + 4 * tile);
+                        ph_cols<ENS_SEQ>(C.m, C.pl, C.m.px.tw32, ws, tile, C.m.B_cols, C.m.B_cols,
+                                         C.m.S[stage == 3 ? 1 : 0], C.m.cpart);
                         if (tile == 0 && tid == 0) {
                             Ctl* gc = C.m.ctl;
                             gc->nf += 1;

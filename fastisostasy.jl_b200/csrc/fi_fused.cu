@@ -166,7 +166,7 @@ k_cols(const Member* __restrict__ mems, const Task* __restrict__ tasks, int B, i
             if (h_gate) cudaGraphSetConditional(h_gate, g);
         }
     }
-    ph_cols(m, hd.plan, m.px.tw32, smem, tk.tile, B, m.S[next_stage == 4 ? 1 : 0], m.cpart + 4 * tk.tile);
+    ph_cols(m, hd.plan, m.px.tw32, smem, tk.tile, B, B, m.S[next_stage == 4 ? 1 : 0], m.cpart);
 }
 
 // ---------------------------------------------------------------------------

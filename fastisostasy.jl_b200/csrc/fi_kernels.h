@@ -62,6 +62,38 @@ const void* persist_kernel(int seqx, int seqy, int minb);
 size_t persist_layout(int nx, int ny, int Mx, int My, int K, int fwd_bytes, int h_rows, int ncols, int B_cols,
                       int h_conv, int B_conv, PersistArgs* a);
 
+// ---- resident step executor (fi_resident.cuh, fi_resident_*.cu) ----
+// Shared-memory offsets (bytes) of the resident kernel; -1: read in place from global memory.
+struct ResLayout {
+    int twx, twy, tice;  // twiddles (twy == twx when the two plans are one), ice times
+    int MS, F;           // moments / transform buffer, and behind it the packed right-hand side;
+                         // together the scratch of the column and convolution phases
+    int P1, P0;          // stage vector and (P0 >= 0) the state, double-buffered, FP64
+    int KA0, KA1;        // k1 / k4 double buffer with halos
+    int KB, KC;          // k2 with halos, k3 own rows
+    int D, visc, ue, dz, Ha, Hb, mult;
+    int chunk;           // own rows per moment pass (even, or the whole tile)
+    int bytes, all;      // all: every optional buffer is in shared memory, the tile in one chunk
+};
+constexpr int RES_MAX_SUB = 8;
+// threads of a block of the resident kernel (res: every buffer resident)
+constexpr int res_threads(int res) { return res ? 512 : ROW_THREADS; }
+struct ResArgs {
+    PersistArgs p;  // h_rows / n_rows, B_cols / n_cols: the resident tiles and their tasks
+    ResLayout L;
+    // the handle's tiles: error-norm partials are kept per h_sub rows (n_part of them) and
+    // corner partials per B_sub columns, so that both sums run in the order of the other
+    // executors; h_rows and B_cols are multiples of them
+    int h_sub, n_part, B_sub, pad_;
+};
+// Fills L for tiles of h rows within `budget` bytes; false when the mandatory buffers do not
+// fit.  grid: blocks of the launch.
+bool res_layout(int nx, int ny, int Mx, int My, int K, int same_plan, int h, int B_cols, int ncols, int h_conv,
+                int B_conv, int grid, size_t budget, ResLayout* L);
+// the kernel with the compiled radix sequences seqx / seqy, or the one that runs the plans'
+// passes, for layouts with all buffers resident or any
+const void* resident_kernel(int seqx, int seqy, int all);
+
 // ---- persistent ensemble executor (fi_ensemble.cu) ----
 constexpr int ENS_MAX_MEMBERS = 256;
 struct EnsArgs {

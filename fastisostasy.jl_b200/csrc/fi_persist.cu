@@ -149,7 +149,7 @@ __device__ __forceinline__ void persist_body(const PersistArgs& a) {
             trace_mark(trace, &tlast, PH_ROWS_FWD2 + 2 * (stage - 2));
             // ---- columns; count the call and evaluate the gate of the next one ----
             for (int tc = bid; tc < a.n_cols; tc += G)
-                ph_cols<SY>(m, pl[1], pl[0].tw32, smem, tc, a.B_cols, Sout, m.cpart + 4 * tc);
+                ph_cols<SY>(m, pl[1], pl[0].tw32, smem, tc, a.B_cols, a.B_cols, Sout, m.cpart);
             if (tid == 0) {
                 sc.nf += 1;
                 if (stage < 4) gate_eval(m, &sc, sc.t + (stage == 2 ? C3 : 1.0) * sc.dt);

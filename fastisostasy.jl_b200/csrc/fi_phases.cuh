@@ -679,11 +679,12 @@ __device__ inline void ph_rows_fwd(const Member& m, const FwdScalars& s, const F
 }
 
 // ---------------------------------------------------------------------------
-// columns (in place on S); cpart_out: this task's 4 corner terms
+// columns (in place on S)
 // ---------------------------------------------------------------------------
+// Bsub: columns per set of corner partials (cpart: the whole array).
 template <int SY = 0>
 __device__ inline void ph_cols(const Member& m, const FftPlan& plan, const float2* twx, unsigned char* ws, int tile,
-                               int B, float2* S, double* cpart_out) {
+                               int B, int Bsub, float2* S, double* cpart) {
     const int ny = m.ny, tid = threadIdx.x, nth = blockDim.x;
     const int kx0 = tile * B;
     const int nb = min(B, m.NH - kx0);
@@ -711,7 +712,11 @@ __device__ inline void ph_cols(const Member& m, const FftPlan& plan, const float
         const int b = i / ny, y = i - b * ny;
         S[(size_t)y * m.sp + kx0 + b] = q[i];
     }
-    if (tid < 4) cpart_out[tid] = column_corner_term(q, ny, m.nx, kx0, nb, twx, tid);
+    if (tid < 4 * ((nb + Bsub - 1) / Bsub)) {
+        const int b0_ = (tid >> 2) * Bsub;
+        cpart[4 * (tile * (B / Bsub)) + tid] =
+            column_corner_term(q + b0_ * ny, ny, m.nx, kx0 + b0_, min(Bsub, nb - b0_), twx, tid & 3);
+    }
     __syncthreads();
 }
 
@@ -828,7 +833,7 @@ __device__ __forceinline__ double partials_sum(const double* part, int n) {
 // together would mix their FP32 rounding (their inputs differ by the cell area, ~1e9).
 // ---------------------------------------------------------------------------
 __device__ inline void ph_conv_rows(const Member& m, const FftPlan& plan, unsigned char* ws, int tile, int h) {
-    const int nx = m.nx, ny = m.ny, Mx = m.Mx, MH = m.MH, tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int nx = m.nx, ny = m.ny, Mx = m.Mx, MH = m.MH, tid = threadIdx.x, tx = tid % TX, ty = tid / TX, nty = blockDim.x / TX;
     const int y0 = tile * h, y1 = min(y0 + h, ny);
     const int np = (y1 - y0 + 1) / 2;
     const int nch = m.elastic_on + m.geoid_on;
@@ -840,7 +845,7 @@ __device__ inline void ph_conv_rows(const Member& m, const FftPlan& plan, unsign
     if (m.geoid_on) { in[cc] = m.sig_geo; out[cc] = m.SB; cc++; }
     const int nt = nch * np;
     float2* zb = (float2*)ws;
-    for (int tr = ty; tr < nt; tr += TY) {
+    for (int tr = ty; tr < nt; tr += nty) {
         const int ch = tr / np, p = tr - ch * np;
         const int ra = y0 + 2 * p;
         const bool hb = ra + 1 < y1;
@@ -852,7 +857,7 @@ __device__ inline void ph_conv_rows(const Member& m, const FftPlan& plan, unsign
     }
     __syncthreads();
     float2* res = fft_batch<false, float>(zb, zb + nt * Mx, plan, nt, Mx);
-    for (int tr = ty; tr < nt; tr += TY) {
+    for (int tr = ty; tr < nt; tr += nty) {
         const int ch = tr / np, p = tr - ch * np;
         const int ra = y0 + 2 * p;
         const bool hb = ra + 1 < y1;
@@ -912,13 +917,13 @@ __device__ inline void ph_conv_cols(const Member& m, const FftPlan& plan, unsign
 // rows, their raw corner values (ue_corner / dz_corner, each double[4]).
 __device__ inline void ph_conv_rows_inv(const Member& m, const FftPlan& plan, unsigned char* ws, int tile, int h, int iue,
                                  double* ue_corner, double* dz_corner) {
-    const int nx = m.nx, ny = m.ny, Mx = m.Mx, MH = m.MH, tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int nx = m.nx, ny = m.ny, Mx = m.Mx, MH = m.MH, tid = threadIdx.x, tx = tid % TX, ty = tid / TX, nty = blockDim.x / TX;
     const int nrow = ny + 2;  // crop rows j1..j1+ny-1, then corner rows 0 and 2ny-2
     const int y0 = tile * h, y1 = min(y0 + h, nrow);
     const int np = (y1 - y0 + 1) / 2;
     if (!m.elastic_on) {
         // RigidLithosphere: ue = 0 (src/deformation.jl:186-189)
-        for (int ry = y0 + ty; ry < min(y1, ny); ry += TY)
+        for (int ry = y0 + ty; ry < min(y1, ny); ry += nty)
             for (int x = tx; x < nx; x += TX) m.ue[iue][ry * nx + x] = 0.0f;
         if (tid == 0 && y1 > ny)
             for (int q = 0; q < 4; q++) ue_corner[q] = 0.0;
@@ -933,7 +938,7 @@ __device__ inline void ph_conv_rows_inv(const Member& m, const FftPlan& plan, un
     if (m.geoid_on) { src[cc] = m.TB; dst[cc] = m.dz; corner[cc] = dz_corner; cc++; }
     const int nt = nch * np;
     float2* zb = (float2*)ws;
-    for (int tr = ty; tr < nt; tr += TY) {
+    for (int tr = ty; tr < nt; tr += nty) {
         const int ch = tr / np, p = tr - ch * np;
         const int ra = y0 + 2 * p;
         const bool hb = ra + 1 < y1;
@@ -949,7 +954,7 @@ __device__ inline void ph_conv_rows_inv(const Member& m, const FftPlan& plan, un
     }
     __syncthreads();
     float2* res = fft_batch<true, float>(zb, zb + nt * Mx, plan, nt, Mx);
-    for (int tr = ty; tr < nt; tr += TY) {
+    for (int tr = ty; tr < nt; tr += nty) {
         const int ch = tr / np, p = tr - ch * np;
         for (int q = 0; q < 2; q++) {
             const int ry = y0 + 2 * p + q;
