@@ -592,8 +592,9 @@ TcOperand opMN(const bf16* p, int ld, long long s = 0, long long s2 = 0) {
     return o;
 }
 
-// C[z] = A[z] B[z]^T over K columns (columns [K1, K) from A2, B2 when K1 > 0)
-template <class Epi>
+// C[z] = A[z] B[z]^T over K columns (columns [K1, K) from A2, B2 when K1 > 0); NTHR 128: 128 x 128
+// tiles of 128 threads, 0: the tile and threads that suit N
+template <int NTHR = 0, class Epi>
 cudaError_t gemm(fi_fno* h, int M, int N, int K, TcOperand A, TcOperand B, int batch, const Epi& epi, int zdiv = 1,
                  TcOperand A2 = TcOperand(), TcOperand B2 = TcOperand(), int K1 = 0) {
     TcGemmArgs g;
@@ -607,9 +608,8 @@ cudaError_t gemm(fi_fno* h, int M, int N, int K, TcOperand A, TcOperand B, int b
     g.K1 = K1;
     g.zdiv = zdiv;
     g.err = h->err;
-    if (N <= 32) return launch_gemm_tc<32>(g, batch, epi, h->st);
-    if (N <= 64) return launch_gemm_tc<64>(g, batch, epi, h->st);
-    return launch_gemm_tc<128>(g, batch, epi, h->st);
+    if constexpr (NTHR == 128) return launch_gemm_tc<128, 128>(g, batch, epi, h->st);
+    else return launch_gemm(g, batch, epi, h->st);
 }
 
 uint64_t splitmix64(uint64_t& s) {
@@ -739,8 +739,9 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
                     B * S, EpiPixAct{lp + SPEC + C * C, h->zs[l], h->vext[l + 1], S, S2, l < NLAYER - 1 ? 1 : 0}, S,
                     opMN(h->vext[l], S2, vs, S), opK(h->Wl + (size_t)l * C * C, C), 2 * KX));
     }
-    FNO_CK(gemm(h, S2, PW, C, opMN(h->vext[NLAYER], S2, vs), opK(h->Q1b, C), B,
-                EpiProj{h->params + o.b1, h->params + o.Q2, h->params + o.b2, y, S2, 0.f}));
+    // one thread sums a row's 128 columns in order: 128 threads
+    FNO_CK(gemm<128>(h, S2, PW, C, opMN(h->vext[NLAYER], S2, vs), opK(h->Q1b, C), B,
+                     EpiProj{h->params + o.b1, h->params + o.Q2, h->params + o.b2, y, S2, 0.f}));
     h->fwdB = B;
     return FI_OK;
 }

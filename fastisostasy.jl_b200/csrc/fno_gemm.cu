@@ -70,9 +70,7 @@ extern "C" int fi_fno_gemm(int32_t M, int32_t N, int32_t K, const void* A, int32
     g.B.mn = bmn;
     g.err = d_err;
     EpiStoreF32 epi{C, ldc, sC};
-    cudaError_t e = N <= 32 ? launch_gemm_tc<32>(g, batch, epi, 0)
-                  : N <= 64 ? launch_gemm_tc<64>(g, batch, epi, 0)
-                            : launch_gemm_tc<128>(g, batch, epi, 0);
+    cudaError_t e = launch_gemm(g, batch, epi, 0);
     int herr = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);

@@ -47,3 +47,24 @@ def test_tc_gemm_mn_major_operands(M, N, K, batch, flags):
     want = torch.bmm(A.float(), B.float().transpose(1, 2)).cuda()
     err = (Cm - want).abs().max().item() / want.abs().max().item()
     assert err < 1e-5, err
+
+
+@pytest.mark.parametrize("M,N,K,batch,fixed", [
+    (128, 32, 64, 2100, "A"), (40, 24, 24, 1900, ""), (100, 64, 32, 1500, "B"), (130, 17, 200, 700, ""),
+    (128, 32, 128, 1000, "B"), (16, 128, 72, 1300, "A"),
+])
+def test_tc_gemm_many_tiles(M, N, K, batch, fixed):
+    """More tiles than blocks: a block walks several, with one or two stage buffers, and copies an
+    operand that is the same for all of them once."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cpu").manual_seed(M + 5 * N + K + batch)
+    A = torch.randn(1 if fixed == "A" else batch, M, K, generator=g).to(torch.bfloat16).cuda()
+    B = torch.randn(1 if fixed == "B" else batch, N, K, generator=g).to(torch.bfloat16).cuda()
+    Cm = torch.full((batch, M, N), float("nan"), dtype=torch.float32, device="cuda")
+    rc = abi.load_library().fi_fno_gemm(M, N, K, C.c_void_p(A.data_ptr()), K, C.c_void_p(B.data_ptr()), K,
+                                        C.c_void_p(Cm.data_ptr()), N, batch, 0 if fixed == "A" else M * K,
+                                        0 if fixed == "B" else N * K, M * N, 0)
+    assert rc == 0
+    want = torch.matmul(A.float(), B.float().transpose(1, 2))
+    err = (Cm - want).abs().max().item() / want.abs().max().item()
+    assert err < 1e-5, err
