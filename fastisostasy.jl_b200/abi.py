@@ -258,6 +258,8 @@ _SIGS = {
     "fi_create": (C.c_int, [C.POINTER(FiConfig), C.POINTER(C.c_void_p)]),
     "fi_set_field": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_size_t]),
     "fi_get_field": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_size_t]),
+    "fi_set_field_rowmajor": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_size_t]),
+    "fi_get_field_rowmajor": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.c_size_t]),
     "fi_set_ice_history": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "fi_set_elastic_table": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "fi_set_channel_scaling": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
@@ -266,6 +268,7 @@ _SIGS = {
     "fi_get_fft_schedule": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "fi_init": (C.c_int, [C.c_void_p]),
     "fi_rhs": (C.c_int, [C.c_void_p, C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
+    "fi_rhs_rowmajor": (C.c_int, [C.c_void_p, C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "fi_rhs_noalloc": (C.c_int, [C.c_void_p, C.c_double, C.c_void_p, C.c_void_p]),
     "fi_run": (C.c_int, [C.c_void_p, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double),
                          C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double),

@@ -57,6 +57,12 @@ struct PlainBufs {
 
 }  // namespace
 
+// the control block with the grid-barrier words of the persistent executors
+struct CtlBar {
+    Ctl c;
+    unsigned int bar[4];
+};
+
 struct fi_handle {
     fi_config cfg;
     std::string err;
@@ -83,6 +89,7 @@ struct fi_handle {
     // fused form
     Member mem{};
     Member* d_mem = nullptr;
+    CtlBar* d_cb = nullptr;  // d_ctl and d_bar point into it
     Ctl* d_ctl = nullptr;
     Task *t_rows = nullptr, *t_cols = nullptr, *t_crow = nullptr, *t_ccol = nullptr, *t_crowi = nullptr;
     int n_rows, n_cols, n_crow, n_ccol, n_crowi;
@@ -498,8 +505,10 @@ static int create_buffers(fi_handle* h) {
         RET(dalloc(h, &GB, (size_t)h->MH * h->My)); m.GB = GB;
         RET(dalloc(h, &m.partial, (size_t)h->ny + 16));
         RET(dalloc(h, &m.cpart, (size_t)4 * (h->NH + 16)));
-        RET(dalloc(h, &h->d_ctl, 1));
-        RET(dalloc(h, &h->d_bar, 4));
+        // the control block and, behind it, the grid-barrier words: one copy moves both
+        RET(dalloc(h, &h->d_cb, 1));
+        h->d_ctl = &h->d_cb->c;
+        h->d_bar = h->d_cb->bar;
         RET(dalloc(h, &h->d_trace, 2 * PH_COUNT));
         m.ctl = h->d_ctl;
         m.tout = h->d_tout;
@@ -619,6 +628,8 @@ static int download(fi_handle* h, std::vector<double>& dst, const T* src, size_t
     return FI_OK;
 }
 
+// h->ctl mirrors the device's control block between calls: every call that runs kernels on it
+// reads it back before it returns.
 static int read_ctl(fi_handle* h) {
     if (h->cfg.form != FI_FORM_FP32) return FI_OK;
     CK(cudaMemcpyAsync(&h->ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, h->stream));
@@ -668,7 +679,40 @@ static double haf_host(double rho_sw_ice, double H, double zb, double zss) {
     return v > 0 ? v : 0.0;
 }
 
-extern "C" int fi_set_field(fi_handle* h, int32_t field, const double* host, size_t n) {
+static dim3 field_grid(const fi_handle* h) { return dim3(cdiv(h->nx, 32), cdiv(h->ny, 32)); }
+
+// an FP64 field on the device to the caller's buffer, through `scratch` when its layout differs
+static int field_to_host(fi_handle* h, const double* src, double* scratch, double* host, int rowmajor) {
+    if (rowmajor) {
+        k_field_out64<<<field_grid(h), dim3(32, 8), 0, h->stream>>>(src, h->nx, h->ny, 1, scratch);
+        CKL();
+        src = scratch;
+    }
+    CK(cudaMemcpyAsync(host, src, N2(h) * 8, cudaMemcpyDeviceToHost, h->stream));
+    return FI_OK;
+}
+
+// the caller's field to dst in the device's layout (through `scratch` when it differs)
+static int field_from_host(fi_handle* h, const double* host, double* scratch, double* dst, int rowmajor) {
+    CK(cudaMemcpyAsync(rowmajor ? scratch : dst, host, N2(h) * 8, cudaMemcpyHostToDevice, h->stream));
+    if (rowmajor) {
+        k_field_in<<<field_grid(h), dim3(32, 8), 0, h->stream>>>(scratch, h->nx, h->ny, 1, dst, nullptr);
+        CKL();
+    }
+    return FI_OK;
+}
+
+// blocked transposition of the caller's (i, j) at i ny + j
+static std::vector<double> from_rowmajor(const fi_handle* h, const double* in) {
+    std::vector<double> v(N2(h));
+    for (int i0 = 0; i0 < h->nx; i0 += 16)
+        for (int j0 = 0; j0 < h->ny; j0 += 16)
+            for (int j = j0; j < std::min(j0 + 16, h->ny); j++)
+                for (int i = i0; i < std::min(i0 + 16, h->nx); i++) v[(size_t)j * h->nx + i] = in[(size_t)i * h->ny + j];
+    return v;
+}
+
+static int set_field(fi_handle* h, int32_t field, const double* host, size_t n, int rowmajor) {
     if (h) cudaSetDevice(h->cfg.device);
     if (!h || !host) return FI_ERR_ARG;
     if (n != N2(h)) return set_err(h, FI_ERR_ARG, "field size %zu != nx*ny", n);
@@ -677,16 +721,25 @@ extern "C" int fi_set_field(fi_handle* h, int32_t field, const double* host, siz
         // caller's buffer (pinned memory makes it one DMA); the next step re-evaluates
         // the FSAL derivative at the new state (u_modified!)
         if (h->cfg.form == FI_FORM_FP32) {
-            RET(read_ctl(h));
-            CK(cudaMemcpyAsync(h->mem.u[h->ctl.ibuf], host, n * 8, cudaMemcpyHostToDevice, h->stream));
+            RET(field_from_host(h, host, h->d_uin, h->mem.u[h->ctl.ibuf], rowmajor));
         } else {
-            CK(cudaMemcpyAsync(h->p.u[h->ctl.ibuf], host, n * 8, cudaMemcpyHostToDevice, h->stream));
+            RET(field_from_host(h, host, h->p.uin, h->p.u[h->ctl.ibuf], rowmajor));
         }
         CK(cudaStreamSynchronize(h->stream));
         if (h->integ_started) h->fsal_pending = true;
         return FI_OK;
     }
-    std::vector<double> v(host, host + n);
+    if (field == FI_FIELD_H_ICE && h->cfg.ice_mode == FI_ICE_EXTERNAL) {
+        const bool f32 = h->cfg.form == FI_FORM_FP32;
+        double* scratch = f32 ? h->d_uin : h->p.uin;
+        CK(cudaMemcpyAsync(scratch, host, n * 8, cudaMemcpyHostToDevice, h->stream));
+        k_field_in<<<field_grid(h), dim3(32, 8), 0, h->stream>>>(scratch, h->nx, h->ny, rowmajor,
+                                                                 f32 ? nullptr : h->p.H, f32 ? h->mem.H_ext : nullptr);
+        CKL();
+        CK(cudaStreamSynchronize(h->stream));
+        return FI_OK;
+    }
+    std::vector<double> v = rowmajor ? from_rowmajor(h, host) : std::vector<double>(host, host + n);
     switch (field) {
         case FI_FIELD_LITHO_RIGIDITY: h->D = v; return FI_OK;
         case FI_FIELD_EFFECTIVE_VISCOSITY: h->eta = v; return FI_OK;
@@ -703,12 +756,16 @@ extern "C" int fi_set_field(fi_handle* h, int32_t field, const double* host, siz
             return FI_OK;
         case FI_FIELD_U: h->u_init = v; h->u_set = true; return FI_OK;
         case FI_FIELD_H_ICE:
-            if (h->cfg.ice_mode != FI_ICE_EXTERNAL)
-                return set_err(h, FI_ERR_ARG, "H_ice is set externally only with FI_ICE_EXTERNAL");
-            if (h->cfg.form == FI_FORM_FP32) return upload(h, h->mem.H_ext, v);
-            return upload(h, h->p.H, v);
+            return set_err(h, FI_ERR_ARG, "H_ice is set externally only with FI_ICE_EXTERNAL");
         default: return set_err(h, FI_ERR_ARG, "field %d is not settable", field);
     }
+}
+
+extern "C" int fi_set_field(fi_handle* h, int32_t field, const double* host, size_t n) {
+    return set_field(h, field, host, n, 0);
+}
+extern "C" int fi_set_field_rowmajor(fi_handle* h, int32_t field, const double* host, size_t n) {
+    return set_field(h, field, host, n, 1);
 }
 
 extern "C" int fi_set_ice_history(fi_handle* h, int32_t K, const double* t, const double* H) {
@@ -1148,43 +1205,50 @@ static int launch_rhs_body(fi_handle* h, int stage, const double* uin, float* vo
 static int rhs_fused(fi_handle* h, int stage, const double* uin, float* vout, double* cout) {
     k_gate<<<1, 32, 0, h->stream>>>(h->d_mem, 1, h->ctl.t_call, 0);
     CKL();
-    RET(launch_sparse(h));
+    // gate_eval's condition on the mirrored control block: no launches for a closed gate
+    const Ctl& c = h->ctl;
+    if (((c.t_call - c.t0) / h->mem.dt_sparse) >= (double)c.count_sparse) RET(launch_sparse(h));
     RET(launch_rhs_body(h, stage, uin, vout, cout, 0, 0));
     return FI_OK;
 }
 
-extern "C" int fi_rhs(fi_handle* h, double t, double* u_inout, double* dudt_out) {
+static int rhs_host(fi_handle* h, double t, double* u_inout, double* dudt_out, int rowmajor) {
     if (h) cudaSetDevice(h->cfg.device);
     if (!h || !u_inout || !dudt_out) return FI_ERR_ARG;
     if (!h->initialized) return set_err(h, FI_ERR_STATE, "fi_init not called");
-    const size_t n = N2(h);
     if (h->cfg.form == FI_FORM_FP32) {
-        RET(read_ctl(h));
         h->ctl.t_call = t;
         h->ctl.status = FI_OK;
-        RET(write_ctl(h));
-        CK(cudaMemcpyAsync(h->d_uin, u_inout, n * 8, cudaMemcpyHostToDevice, h->stream));
+        CK(cudaMemcpyAsync(h->d_ctl, &h->ctl, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
+        // the other state buffer is free until the call writes u there
+        double* const other = h->mem.u[h->ctl.ibuf ^ 1];
+        RET(field_from_host(h, u_inout, other, h->d_uin, rowmajor));
         RET(rhs_fused(h, 0, h->d_uin, h->d_vscr, h->d_cscr));
         RET(read_ctl(h));
         if (h->ctl.status) return set_err(h, h->ctl.status, "%s", fi_status_string(h->ctl.status));
-        std::vector<float> v(n);
-        double cc[4];
-        CK(cudaMemcpyAsync(u_inout, h->mem.u[h->ctl.ibuf ^ 1], n * 8, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaMemcpyAsync(v.data(), h->d_vscr, n * 4, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaMemcpyAsync(cc, h->d_cscr, 32, cudaMemcpyDeviceToHost, h->stream));
+        RET(field_to_host(h, other, h->d_uin, u_inout, rowmajor));
+        k_field_out32<<<field_grid(h), dim3(32, 8), 0, h->stream>>>(h->d_vscr, h->d_cscr, h->cfg.bc_viscous_border, 0.0,
+                                                                    h->nx, h->ny, rowmajor, h->d_uin);
+        CKL();
+        CK(cudaMemcpyAsync(dudt_out, h->d_uin, N2(h) * 8, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
-        const double off = corner_mean(cc) - h->cfg.bc_viscous_border;
-        for (size_t k = 0; k < n; k++) dudt_out[k] = (double)v[k] - off;
     } else {
-        CK(cudaMemcpyAsync(h->p.uin, u_inout, n * 8, cudaMemcpyHostToDevice, h->stream));
+        RET(field_from_host(h, u_inout, h->p.tmp, h->p.uin, rowmajor));
         RET(rhs_plain(h, t, h->p.uin, h->p.fscratch));
-        CK(cudaMemcpyAsync(u_inout, h->p.uin, n * 8, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaMemcpyAsync(dudt_out, h->p.fscratch, n * 8, cudaMemcpyDeviceToHost, h->stream));
+        RET(field_to_host(h, h->p.uin, h->p.tmp, u_inout, rowmajor));
+        RET(field_to_host(h, h->p.fscratch, h->p.tmp, dudt_out, rowmajor));
         CK(cudaStreamSynchronize(h->stream));
     }
     h->last_call = 1;
     h->last_rhs_t = t;
     return FI_OK;
+}
+
+extern "C" int fi_rhs(fi_handle* h, double t, double* u_inout, double* dudt_out) {
+    return rhs_host(h, t, u_inout, dudt_out, 0);
+}
+extern "C" int fi_rhs_rowmajor(fi_handle* h, double t, double* u_inout, double* dudt_out) {
+    return rhs_host(h, t, u_inout, dudt_out, 1);
 }
 
 static_assert((size_t)FI_NOALLOC_MAX_CELLS == NOALLOC_MAX_CELLS, "scratch limit mismatch");
@@ -1769,7 +1833,6 @@ static int persist_fn(fi_handle* h, const void** out) {
 static int run_segment_persist(fi_handle* h) {
     const void* kfn = nullptr;
     RET(persist_fn(h, &kfn));
-    CK(cudaMemsetAsync(h->d_bar, 0, 4 * sizeof(unsigned int), h->stream));
     const long long gp = g_grid_polls.load();
     h->pargs.polls = gp >= 0 ? gp : PERSIST_SPIN_LIMIT;
     h->pargs.bar_extra = (unsigned)g_grid_extra.load();
@@ -1780,10 +1843,11 @@ static int run_segment_persist(fi_handle* h) {
     CK(cudaLaunchCooperativeKernel(kfn, dim3(h->resident ? h->resident_grid : h->persist_grid),
                                    dim3(h->resident ? res_threads(h->rargs.L.all) : ROW_THREADS), args,
                                    h->resident ? h->resident_smem : h->persist_smem, h->stream));
-    unsigned int bar[4];
-    CK(cudaMemcpyAsync(bar, h->d_bar, sizeof(bar), cudaMemcpyDeviceToHost, h->stream));
-    RET(read_ctl(h));
-    if (bar[2]) return set_err(h, FI_ERR_TIMEOUT, "persistent step kernel: a grid barrier wait gave up");
+    CtlBar cb;
+    CK(cudaMemcpyAsync(&cb, h->d_cb, sizeof(cb), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    h->ctl = cb.c;
+    if (cb.bar[2]) return set_err(h, FI_ERR_TIMEOUT, "persistent step kernel: a grid barrier wait gave up");
     return FI_OK;
 }
 
@@ -1885,9 +1949,8 @@ static int run_segment_plain(fi_handle* h) {
 // FSAL re-evaluation after a modifying callback: k1 = f(u, t)
 static int reeval_fsal(fi_handle* h) {
     if (h->cfg.form == FI_FORM_FP32) {
-        RET(read_ctl(h));
         h->ctl.t_call = h->ctl.t;
-        RET(write_ctl(h));
+        CK(cudaMemcpyAsync(h->d_ctl, &h->ctl, sizeof(Ctl), cudaMemcpyHostToDevice, h->stream));
         RET(rhs_fused(h, 1, nullptr, nullptr, nullptr));
         RET(read_ctl(h));
     } else {
@@ -2006,10 +2069,13 @@ static int solve_until_(fi_handle* h, const OutBufs* o) {
             h->fsal_pending = false;
             if (h->ctl.status != FI_OK) return set_err(h, h->ctl.status, "%s", fi_status_string(h->ctl.status));
         }
-        if (fused) RET(read_ctl(h));
         h->ctl.t_stop = h->tstops.front();
-        if (fused) RET(write_ctl(h));
-        if (fused) RET(run_segment_fused(h)); else RET(run_segment_plain(h));
+        if (fused) {
+            // with cleared barrier words; the segment ends with a wait, so `cb` outlives the copy
+            CtlBar cb{h->ctl, {0, 0, 0, 0}};
+            CK(cudaMemcpyAsync(h->d_cb, &cb, sizeof(cb), cudaMemcpyHostToDevice, h->stream));
+            RET(run_segment_fused(h));
+        } else RET(run_segment_plain(h));
         h->segments += 1;
         Ctl& ct = h->ctl;
         if (ct.status != FI_OK)
@@ -2081,7 +2147,6 @@ extern "C" int fi_step(fi_handle* h, double dt) {
     if (h) cudaSetDevice(h->cfg.device);
     if (!h || !(dt > 0)) return FI_ERR_ARG;
     if (!h->integ_started) return set_err(h, FI_ERR_STATE, "fi_init_integrator not called");
-    if (h->cfg.form == FI_FORM_FP32) RET(read_ctl(h));
     const double next_t = h->ctl.t + dt;
     if (next_t > h->cfg.t1) return set_err(h, FI_ERR_ARG, "step beyond t_span");
     // add_tstop!(integrator, t + dt); advance until t >= next_t
@@ -2202,6 +2267,10 @@ struct fi_ensemble {
     unsigned int* d_bar = nullptr;
     unsigned long long* d_counter = nullptr;
     unsigned long long* d_trace = nullptr;
+    Ctl* d_gather = nullptr;      // all members' control blocks, for one copy
+    double* d_t_stop = nullptr;   // their segment ends
+    std::vector<Ctl> gather;
+    std::vector<double> t_stop;
     EnsArgs args{};
     const void* kfn = nullptr;  // the ensemble kernel build (ens_kernel)
     int grid = 0;
@@ -2215,10 +2284,14 @@ static void ensemble_free(fi_ensemble* e) {
     if (e->d_bar) cudaFree(e->d_bar);
     if (e->d_counter) cudaFree(e->d_counter);
     if (e->d_trace) cudaFree(e->d_trace);
+    if (e->d_gather) cudaFree(e->d_gather);
+    if (e->d_t_stop) cudaFree(e->d_t_stop);
     if (e->e0) cudaEventDestroy(e->e0);
     if (e->e1) cudaEventDestroy(e->e1);
     if (e->stream) cudaStreamDestroy(e->stream);
     e->d_mems = nullptr; e->d_ctls = nullptr; e->d_bar = nullptr; e->d_counter = nullptr; e->d_trace = nullptr;
+    e->d_gather = nullptr;
+    e->d_t_stop = nullptr;
     e->e0 = e->e1 = nullptr;
     e->stream = nullptr;
 }
@@ -2257,6 +2330,8 @@ static bool ensemble_setup_persist(fi_ensemble* e) {
                      cudaMalloc(&e->d_ctls, n * sizeof(Ctl*)) == cudaSuccess &&
                      cudaMalloc(&e->d_bar, 4 * sizeof(unsigned int)) == cudaSuccess &&
                      cudaMalloc(&e->d_counter, sizeof(unsigned long long)) == cudaSuccess &&
+                     cudaMalloc(&e->d_gather, n * sizeof(Ctl)) == cudaSuccess &&
+                     cudaMalloc(&e->d_t_stop, n * sizeof(double)) == cudaSuccess &&
                      cudaMalloc(&e->d_trace, 2 * PH_COUNT * sizeof(unsigned long long)) == cudaSuccess &&
                      cudaMemcpy(e->d_mems, hm.data(), n * sizeof(Member), cudaMemcpyHostToDevice) == cudaSuccess &&
                      cudaMemcpy(e->d_ctls, hc.data(), n * sizeof(Ctl*), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -2319,9 +2394,8 @@ void fi_ensemble_destroy(fi_ensemble* e) {
     delete e;
 }
 
-// One member's completion of a launched segment (the tail of solve_until_).
+// One member's completion of a launched segment (the tail of solve_until_), its control block read.
 static int ensemble_finish_segment(fi_handle* h) {
-    RET(read_ctl(h));
     h->segments += 1;
     Ctl& ct = h->ctl;
     if (ct.status != FI_OK)
@@ -2350,6 +2424,20 @@ static int ensemble_launch_segment(fi_handle* h) {
     return launch_segment_graph_async(h);
 }
 
+// every member's control block into its host mirror, by one copy; waits for the ensemble's stream
+static cudaError_t ensemble_read_ctls(fi_ensemble* e) {
+    const int n = (int)e->mem.size();
+    e->gather.resize(n);
+    k_ens_gather<<<n, 128, 0, e->stream>>>(e->d_ctls, n, e->d_gather);
+    cudaError_t ce = cudaGetLastError();
+    if (ce == cudaSuccess)
+        ce = cudaMemcpyAsync(e->gather.data(), e->d_gather, n * sizeof(Ctl), cudaMemcpyDeviceToHost, e->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+    if (ce == cudaSuccess)
+        for (int i = 0; i < n; i++) e->mem[i]->ctl = e->gather[i];
+    return ce;
+}
+
 // Persistent path of fi_ensemble_step: each launch runs one segment of every member
 // that has one left; members are prepared (FSAL, t_stop) and finished on the host.
 static int ensemble_step_persist(fi_ensemble* e, std::vector<std::vector<double>>& rest, std::vector<int>& st,
@@ -2368,28 +2456,26 @@ static int ensemble_step_persist(fi_ensemble* e, std::vector<std::vector<double>
                 h->fsal_pending = false;
                 if (!rc && h->ctl.status != FI_OK) rc = set_err(h, h->ctl.status, "%s", fi_status_string(h->ctl.status));
             }
-            if (!rc) rc = read_ctl(h);
-            if (!rc) {
-                h->ctl.t_stop = h->tstops.front();
-                rc = write_ctl(h);
-            }
             if (rc) { st[i] = rc; state[i] = 2; continue; }
+            h->ctl.t_stop = h->tstops.front();
             state[i] = 1;
             any = true;
         }
-        // members without a segment in this ensemble step must not step: their t_stop is their t
-        for (int i = 0; i < n; i++) {
-            if (state[i] == 1) continue;
-            fi_handle* h = e->mem[i];
-            if (read_ctl(h) == FI_OK) {
-                h->ctl.t_stop = h->ctl.t;
-                write_ctl(h);
-            }
-        }
         if (!any) break;
-        if (cudaMemsetAsync(e->d_bar, 0, 4 * sizeof(unsigned int), e->stream) != cudaSuccess ||
+        // members without a segment in this ensemble step must not step: their t_stop is their t.
+        // (Every call that works on a member's own stream waits for it before it returns.)
+        e->t_stop.resize(n);
+        for (int i = 0; i < n; i++) {
+            Ctl& ct = e->mem[i]->ctl;
+            if (state[i] != 1) ct.t_stop = ct.t;
+            e->t_stop[i] = ct.t_stop;
+        }
+        if (cudaMemcpyAsync(e->d_t_stop, e->t_stop.data(), n * sizeof(double), cudaMemcpyHostToDevice, e->stream) !=
+                cudaSuccess ||
+            cudaMemsetAsync(e->d_bar, 0, 4 * sizeof(unsigned int), e->stream) != cudaSuccess ||
             cudaMemsetAsync(e->d_counter, 0, sizeof(unsigned long long), e->stream) != cudaSuccess)
             return FI_ERR_CUDA;
+        k_ens_t_stop<<<cdiv(n, 128), 128, 0, e->stream>>>(e->d_ctls, n, e->d_t_stop);
         void* args[] = {(void*)&e->args};
         cudaEventRecord(e->e0, e->stream);
         cudaError_t ce = cudaLaunchCooperativeKernel(e->kfn, dim3(e->grid), dim3(ROW_THREADS), args,
@@ -2397,7 +2483,7 @@ static int ensemble_step_persist(fi_ensemble* e, std::vector<std::vector<double>
         cudaEventRecord(e->e1, e->stream);
         unsigned int bar[4] = {0, 0, 0, 0};
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(bar, e->d_bar, sizeof(bar), cudaMemcpyDeviceToHost, e->stream);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
+        if (ce == cudaSuccess) ce = ensemble_read_ctls(e);
         if (ce != cudaSuccess) {
             for (int i = 0; i < n; i++)
                 if (state[i] == 1) {
@@ -2438,15 +2524,15 @@ extern "C" int fi_ensemble_step(fi_ensemble* e, double dt, int32_t* status) {
     std::vector<int> st(n, FI_OK), state(n, 0);  // state: 0 idle, 1 launched, 2 done
     for (int i = 0; i < n; i++) {
         fi_handle* h = e->mem[i];
-        int rc = read_ctl(h);
+        int rc = FI_OK;
         const double next_t = h->ctl.t + dt;
-        if (!rc && next_t > h->cfg.t1) rc = set_err(h, FI_ERR_ARG, "step beyond t_span");
+        if (next_t > h->cfg.t1) rc = set_err(h, FI_ERR_ARG, "step beyond t_span");
         if (rc) { st[i] = rc; state[i] = 2; continue; }
         std::vector<double>& v = h->tstops;
         v.insert(std::lower_bound(v.begin(), v.end(), next_t), next_t);
         v.erase(std::unique(v.begin(), v.end()), v.end());
         while (!v.empty() && v.back() > next_t) { rest[i].insert(rest[i].begin(), v.back()); v.pop_back(); }
-        if (cudaEventRecord(e->ev_start[i], h->stream) != cudaSuccess) { st[i] = FI_ERR_CUDA; state[i] = 2; }
+        if (!e->persist && cudaEventRecord(e->ev_start[i], h->stream) != cudaSuccess) { st[i] = FI_ERR_CUDA; state[i] = 2; }
     }
     if (e->persist) return ensemble_step_persist(e, rest, st, state, status);
     for (;;) {
@@ -2463,7 +2549,8 @@ extern "C" int fi_ensemble_step(fi_ensemble* e, double dt, int32_t* status) {
         if (!any) break;
         for (int i = 0; i < n; i++) {
             if (state[i] != 1) continue;
-            const int rc = ensemble_finish_segment(e->mem[i]);
+            int rc = read_ctl(e->mem[i]);
+            if (!rc) rc = ensemble_finish_segment(e->mem[i]);
             state[i] = rc ? 2 : 0;
             if (rc) st[i] = rc;
         }
@@ -2604,7 +2691,7 @@ extern "C" int fi_time_kernels(fi_handle* h, int32_t reps, double* ms) {
         CK(cudaEventElapsedTime(&t, h->ev0, h->ev1));
         ms[k] = (double)t / reps;
     }
-    return FI_OK;
+    return read_ctl(h);
 }
 
 static_assert(FI_NUM_PHASES == PH_COUNT, "phase count mismatch");
@@ -2633,13 +2720,44 @@ extern "C" int fi_get_phase_trace(fi_handle* h, double* ms, int64_t* counts) {
     return FI_OK;
 }
 
-extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n) {
+static int get_field(fi_handle* h, int32_t field, double* host, size_t n, int rowmajor) {
     if (h) cudaSetDevice(h->cfg.device);
     if (!h || !host) return FI_ERR_ARG;
     if (n != N2(h)) return set_err(h, FI_ERR_ARG, "field size %zu != nx*ny", n);
     std::vector<double> v;
     const fi_config& c = h->cfg;
     const bool fused = c.form == FI_FORM_FP32;
+    if (h->initialized && (field == FI_FIELD_U || field == FI_FIELD_UE || field == FI_FIELD_DUDT ||
+                           field == FI_FIELD_DZ_SS)) {
+        // the fields a coupled model reads after each step: converted on the device, one copy
+        if (!fused) {
+            const PlainBufs& p = h->p;
+            const double* src = field == FI_FIELD_U ? p.now_u : field == FI_FIELD_UE ? p.ue
+                                : field == FI_FIELD_DUDT ? p.dudt : p.dz;
+            RET(field_to_host(h, src, p.uin, host, rowmajor));
+        } else {
+            const Member& m = h->mem;
+            const Ctl& ct = h->ctl;
+            const bool scr = h->last_call == 1;
+            if (field == FI_FIELD_U) {
+                RET(field_to_host(h, m.u[scr ? ct.ibuf ^ 1 : ct.ibuf], h->d_uin, host, rowmajor));
+            } else {
+                const float* src = field == FI_FIELD_UE ? m.ue[ct.iue] : field == FI_FIELD_DZ_SS ? m.dz
+                                   : scr ? h->d_vscr : m.k14[ct.ik];
+                const double* c4 = field == FI_FIELD_DUDT && scr ? h->d_cscr : nullptr;
+                const double border = field == FI_FIELD_UE ? c.bc_elastic_border
+                                      : field == FI_FIELD_DUDT ? c.bc_viscous_border : c.bc_sea_surface_border;
+                const double off = corner_mean(field == FI_FIELD_UE ? ct.ue_corner[ct.iue]
+                                               : field == FI_FIELD_DUDT ? ct.kcorner[ct.ik] : ct.dz_corner) - border;
+                k_field_out32<<<field_grid(h), dim3(32, 8), 0, h->stream>>>(src, c4, border, off, h->nx, h->ny,
+                                                                            rowmajor, h->d_uin);
+                CKL();
+                CK(cudaMemcpyAsync(host, h->d_uin, n * 8, cudaMemcpyDeviceToHost, h->stream));
+            }
+        }
+        CK(cudaStreamSynchronize(h->stream));
+        return FI_OK;
+    }
     switch (field) {
         case FI_FIELD_LITHO_RIGIDITY: v = h->D; break;
         case FI_FIELD_EFFECTIVE_VISCOSITY: v = h->eta; break;
@@ -2662,10 +2780,6 @@ extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n)
                 const PlainBufs& p = h->p;
                 const double* src = nullptr;
                 switch (field) {
-                    case FI_FIELD_U: src = p.now_u; break;
-                    case FI_FIELD_UE: src = p.ue; break;
-                    case FI_FIELD_DUDT: src = p.dudt; break;
-                    case FI_FIELD_DZ_SS: src = p.dz; break;
                     case FI_FIELD_H_ICE: src = p.H; break;
                     case FI_FIELD_Z_SS: src = p.z_ss; break;
                     case FI_FIELD_Z_B: src = p.z_b; break;
@@ -2683,30 +2797,7 @@ extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n)
                 break;
             }
             const Member& m = h->mem;
-            std::vector<double> ue, dz;
-            RET(download(h, ue, m.ue[ct.iue], n));
-            const double cue = corner_mean(ct.ue_corner[ct.iue]) - c.bc_elastic_border;
-            for (auto& x : ue) x -= cue;
-            RET(download(h, dz, m.dz, n));
-            const double cdz = corner_mean(ct.dz_corner) - c.bc_sea_surface_border;
-            for (auto& x : dz) x -= cdz;
             switch (field) {
-                case FI_FIELD_U: RET(download(h, v, m.u[h->last_call == 1 ? ct.ibuf ^ 1 : ct.ibuf], n)); break;
-                case FI_FIELD_UE: v = ue; break;
-                case FI_FIELD_DZ_SS: v = dz; break;
-                case FI_FIELD_DUDT: {
-                    const bool scr = h->last_call == 1;
-                    RET(download(h, v, scr ? h->d_vscr : m.k14[ct.ik], n));
-                    double cc[4];
-                    if (scr) {
-                        CK(cudaMemcpy(cc, h->d_cscr, 32, cudaMemcpyDeviceToHost));
-                    } else {
-                        memcpy(cc, ct.kcorner[ct.ik], 32);
-                    }
-                    const double off = corner_mean(cc) - c.bc_viscous_border;
-                    for (auto& x : v) x -= off;
-                    break;
-                }
                 case FI_FIELD_H_ICE: {
                     int st;
                     interp_ice_host(h, h->last_call == 1 ? h->last_rhs_t : ct.t, v, &st);
@@ -2714,9 +2805,14 @@ extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n)
                     break;
                 }
                 case FI_FIELD_Z_SS:
+                {
+                    std::vector<double> dz;
+                    RET(download(h, dz, m.dz, n));
+                    const double cdz = corner_mean(ct.dz_corner) - c.bc_sea_surface_border;
                     v.resize(n);
-                    for (size_t k = 0; k < n; k++) v[k] = h->z_ss_ref[k] + dz[k] + ct.z_bsl;
+                    for (size_t k = 0; k < n; k++) v[k] = h->z_ss_ref[k] + (dz[k] - cdz) + ct.z_bsl;
                     break;
+                }
                 case FI_FIELD_MASKGROUNDED: RET(download(h, v, m.mgr, n)); break;
                 case FI_FIELD_MASKOCEAN: RET(download(h, v, m.moc, n)); break;
                 case FI_FIELD_H_WATER: RET(download(h, v, m.hwater, n)); break;
@@ -2731,8 +2827,22 @@ extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n)
             }
         }
     }
-    memcpy(host, v.data(), n * sizeof(double));
+    if (!rowmajor) {
+        memcpy(host, v.data(), n * sizeof(double));
+        return FI_OK;
+    }
+    for (int j0 = 0; j0 < h->ny; j0 += 16)
+        for (int i0 = 0; i0 < h->nx; i0 += 16)
+            for (int i = i0; i < std::min(i0 + 16, h->nx); i++)
+                for (int j = j0; j < std::min(j0 + 16, h->ny); j++) host[(size_t)i * h->ny + j] = v[(size_t)j * h->nx + i];
     return FI_OK;
+}
+
+extern "C" int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n) {
+    return get_field(h, field, host, n, 0);
+}
+extern "C" int fi_get_field_rowmajor(fi_handle* h, int32_t field, double* host, size_t n) {
+    return get_field(h, field, host, n, 1);
 }
 
 // ---------------------------------------------------------------------------

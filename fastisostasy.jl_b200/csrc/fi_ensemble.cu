@@ -378,6 +378,16 @@ __global__ void __launch_bounds__(RT, 2) k_ens(EnsArgs a) {
     if (!ok && tid == 0) atomicExch(a.bar + 2, 1u);
 }
 
+// Control blocks of all members to / from one array (one copy instead of one per member): their
+// contents, and the segment end of each member.
+__global__ void k_ens_gather(Ctl* const* ctls, int n, Ctl* out) {
+    if ((int)blockIdx.x < n) copy_words(out + blockIdx.x, ctls[blockIdx.x], sizeof(Ctl));
+}
+__global__ void k_ens_t_stop(Ctl* const* ctls, int n, const double* t_stop) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) ctls[i]->t_stop = t_stop[i];
+}
+
 // Shared-memory layout: [phase workspace][one twiddle table][ice times]
 size_t ens_layout(const Member* host_mems, int n, EnsArgs* a) {
     size_t ws = 0;

@@ -111,6 +111,8 @@ struct EnsArgs {
 // grids where a member's schedule has one, 0 always the plans' runtime passes
 const void* ens_kernel(int dispatch);
 size_t ens_layout(const Member* host_mems, int n, EnsArgs* a);
+__global__ void k_ens_gather(Ctl* const* ctls, int n, Ctl* out);
+__global__ void k_ens_t_stop(Ctl* const* ctls, int n, const double* t_stop);
 
 // ---- FP64 transforms and set-up (fi_setup.cu) ----
 __global__ void k_fft64_rows(double2* a, int nx, int ny, int pitch, const FftPlan* plans, int plan, int inverse,

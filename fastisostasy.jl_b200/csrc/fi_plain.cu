@@ -306,4 +306,62 @@ __global__ void k_out_stage(const double* u, const float* ue, double cue, const 
     }
 }
 
+// ---------------------------------------------------------------------------
+// fields between the device's layout ((i, j) at i + j nx) and the caller's
+// ---------------------------------------------------------------------------
+// out(i, j) = in(i, j) - (corner mean of c4 - border) (c4 null: - off), FP64; rowmajor: (i, j) of
+// out at i ny + j, through a 32 x 32 tile so that both sides are read and written along rows.
+template <typename T>
+__device__ __forceinline__ void field_out(const T* in, const double* c4, double border, double off, int nx, int ny,
+                                          int rowmajor, double* out) {
+    __shared__ double tile[32][33];
+    if (c4) off = (0.25 * (c4[0] + c4[1] + c4[2] + c4[3])) - border;
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + threadIdx.x, j = j0 + r;
+        if (i < nx && j < ny) {
+            const double v = (double)in[(size_t)j * nx + i] - off;
+            if (rowmajor) tile[r][threadIdx.x] = v;
+            else out[(size_t)j * nx + i] = v;
+        }
+    }
+    if (!rowmajor) return;
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + r, j = j0 + threadIdx.x;
+        if (i < nx && j < ny) out[(size_t)i * ny + j] = tile[threadIdx.x][r];
+    }
+}
+__global__ void k_field_out64(const double* in, int nx, int ny, int rowmajor, double* out) {
+    field_out(in, nullptr, 0.0, 0.0, nx, ny, rowmajor, out);
+}
+__global__ void k_field_out32(const float* in, const double* c4, double border, double off, int nx, int ny,
+                              int rowmajor, double* out) {
+    field_out(in, c4, border, off, nx, ny, rowmajor, out);
+}
+
+// in(i, j) at i ny + j (rowmajor) or i + j nx -> the device's layout, FP64 and / or FP32
+__global__ void k_field_in(const double* in, int nx, int ny, int rowmajor, double* out64, float* out32) {
+    __shared__ double tile[32][33];
+    const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        if (rowmajor) {
+            const int i = i0 + r, j = j0 + threadIdx.x;
+            if (i < nx && j < ny) tile[threadIdx.x][r] = in[(size_t)i * ny + j];
+        } else {
+            const int i = i0 + threadIdx.x, j = j0 + r;
+            if (i < nx && j < ny) tile[r][threadIdx.x] = in[(size_t)j * nx + i];
+        }
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        const int i = i0 + threadIdx.x, j = j0 + r;
+        if (i < nx && j < ny) {
+            const double v = tile[r][threadIdx.x];
+            if (out64) out64[(size_t)j * nx + i] = v;
+            if (out32) out32[(size_t)j * nx + i] = (float)v;
+        }
+    }
+}
+
 }  // namespace fi

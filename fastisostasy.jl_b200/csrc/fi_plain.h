@@ -53,6 +53,10 @@ __global__ void kp_lc_in(const double* s_load, const double* s_l, double g, cons
 __global__ void kp_lc_step(double2* U, const double2* F, const double* eta, const double* pd, const double* R,
                            const double* D, double rho_m_g, double dt, size_t n);
 __global__ void kp_real(const double2* U, double* u, size_t n);
+__global__ void k_field_out64(const double* in, int nx, int ny, int rowmajor, double* out);
+__global__ void k_field_out32(const float* in, const double* c4, double border, double off, int nx, int ny,
+                              int rowmajor, double* out);
+__global__ void k_field_in(const double* in, int nx, int ny, int rowmajor, double* out64, float* out32);
 __global__ void k_out_stage(const double* u, const float* ue, double cue, const float* dudt, double cdu,
                             const float* dz, double cdz, double* out, size_t n);
 }  // namespace fi

@@ -627,14 +627,21 @@ class Simulation:
 
     def set_field(self, name, arr):
         self._ensure_handle()
-        buf = to_c(arr)
-        self._check(self.lib.fi_set_field(self._handle, abi.FIELDS[name], abi.dptr(buf), buf.size), f"set {name}")
+        a = np.asarray(arr, dtype=np.float64)
+        if a.shape == (self.domain.nx, self.domain.ny) and a.flags.c_contiguous:
+            # numpy's layout as it is: the library changes it on the device
+            rc = self.lib.fi_set_field_rowmajor(self._handle, abi.FIELDS[name], abi.dptr(a.reshape(-1)), a.size)
+        else:
+            buf = to_c(a)
+            rc = self.lib.fi_set_field(self._handle, abi.FIELDS[name], abi.dptr(buf), buf.size)
+        self._check(rc, f"set {name}")
 
     def get_field(self, name):
         self._ensure_handle()
-        buf = np.empty(self.domain.nx * self.domain.ny)
-        self._check(self.lib.fi_get_field(self._handle, abi.FIELDS[name], abi.dptr(buf), buf.size), f"get {name}")
-        return from_c(buf, self.domain.nx, self.domain.ny)
+        buf = np.empty((self.domain.nx, self.domain.ny))
+        self._check(self.lib.fi_get_field_rowmajor(self._handle, abi.FIELDS[name], abi.dptr(buf.reshape(-1)), buf.size),
+                    f"get {name}")
+        return buf
 
     def init_problem(self):
         """Reference state + init_problem! (src/simulation.jl:305-312)."""
@@ -720,6 +727,12 @@ def update_diagnostics(dudt, u, sim: Simulation, t):
     """update_diagnostics!(dudt, u, sim, t): one RHS evaluation; u and dudt are
     (nx, ny) float64 arrays updated in place."""
     sim.init_problem()
+    if all(isinstance(a, np.ndarray) and a.dtype == np.float64 and a.shape == (sim.domain.nx, sim.domain.ny)
+           and a.flags.c_contiguous and a.flags.aligned and a.flags.writeable for a in (u, dudt)) \
+            and not np.shares_memory(u, dudt):
+        sim._check(sim.lib.fi_rhs_rowmajor(sim._handle, float(t), abi.dptr(u.reshape(-1)), abi.dptr(dudt.reshape(-1))),
+                   "fi_rhs")
+        return
     ub = to_c(u)
     db = np.empty_like(ub)
     sim._check(sim.lib.fi_rhs(sim._handle, float(t), abi.dptr(ub), abi.dptr(db)), "fi_rhs")

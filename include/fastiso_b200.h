@@ -206,6 +206,10 @@ int fi_create(const fi_config* cfg, fi_handle** out);
 /* Copy a host field (nx*ny doubles) to / from the device. */
 int fi_set_field(fi_handle* h, int32_t field, const double* host, size_t n);
 int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n);
+/* The same for callers whose arrays are row-major (element (i,j) at j + i*ny, as numpy's
+ * (nx, ny) arrays): the layout changes on the device, in the copy's shadow. */
+int fi_set_field_rowmajor(fi_handle* h, int32_t field, const double* host, size_t n);
+int fi_get_field_rowmajor(fi_handle* h, int32_t field, double* host, size_t n);
 
 /* TimeInterpolatedIceThickness(t_vec, H_vec, domain) -- src/boundary_conditions.jl:36-40.
  * K snapshots, H is K*nx*ny doubles, t strictly increasing. */
@@ -260,6 +264,8 @@ int fi_init(fi_handle* h);
  * state (sparse update gate, column anomalies).  u is modified in place by the
  * viscous corner boundary condition exactly as in the reference. */
 int fi_rhs(fi_handle* h, double t, double* u_inout, double* dudt_out);
+/* fi_rhs on row-major arrays (see fi_set_field_rowmajor) */
+int fi_rhs_rowmajor(fi_handle* h, double t, double* u_inout, double* dudt_out);
 
 /* No counterpart in the reference: fi_rhs for callers that may not allocate
  * memory, e.g. a coupled ice-sheet model that keeps its state in device
