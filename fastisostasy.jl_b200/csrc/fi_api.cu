@@ -577,6 +577,10 @@ static int create_buffers(fi_handle* h) {
         const size_t s1 = fft64_rows_smem(std::max(h->nx, h->Mx), 1), s2 = fft64_cols_smem(std::max(h->ny, h->My), 1);
         CK(cudaFuncSetAttribute(k_fft64_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
         CK(cudaFuncSetAttribute(k_fft64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
+        const size_t r1 = fft64_rows_smem(h->nx, 1), r2 = fft64_cols_smem(h->ny, 1);
+        CK(cudaFuncSetAttribute(kp_div_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r1));
+        CK(cudaFuncSetAttribute(kp_rows_real, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r1));
+        CK(cudaFuncSetAttribute(kp_spec_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2));
     }
     if (h->cfg.form == FI_FORM_FP32) {
         // FP64 transforms of the set-up are needed by both forms
@@ -917,7 +921,7 @@ static std::vector<double> viscous_green(const fi_handle* h) {
 static int rhs_fused(fi_handle* h, int stage, const double* uin, float* vout, double* cout);
 static int setup_persist(fi_handle* h, int K);
 static int plan_layouts(fi_handle* h, int K);
-static int rhs_plain(fi_handle* h, double t, double* u, double* dudt);
+static int rhs_plain(fi_handle* h, double t, double* u, double* dudt, const PlainStage* stage = nullptr);
 
 extern "C" int fi_init(fi_handle* h) {
     if (h) cudaSetDevice(h->cfg.device);
@@ -1319,21 +1323,21 @@ static int conv_plain(fi_handle* h, const double* input, const double2* Ghat, do
 // update_diagnostics!(dudt, u, sim, t), one kernel per broadcast of the reference
 static int reduce_host(fi_handle* h, const double* d_partial, int nblk, int stride, double* out);
 
-static int rhs_plain(fi_handle* h, double t, double* u, double* dudt) {
+// The right-hand side at u (stage null), or at a stage vector that u receives.
+static int rhs_plain(fi_handle* h, double t, double* u, double* dudt, const PlainStage* stage) {
     const fi_config& c = h->cfg;
     PlainBufs& p = h->p;
     const size_t n = N2(h);
     const int nx = h->nx, ny = h->ny;
     const int g = gs(n);
     h->nf_plain += 1;
-    RET(corner_bc_plain(h, u, nx, ny, c.bc_viscous_border));
-    kp_bedrock<<<g, NT, 0, h->stream>>>(u, p.ue, p.z_b_ref, p.u_ref, p.now_u, p.z_b, p.s_m, c.rho_uppermantle, n);
-    CKL();
+    const double *Ha = nullptr, *Hb = nullptr;
+    int exact = 1;
+    double dti = 1.0, ts = 0.0;
     if (c.ice_mode == FI_ICE_TIME_INTERPOLATED) {
         const std::vector<double>& tt = h->ice_t;
         const int K = (int)tt.size();
-        int i = 0, exact = 1;
-        double dti = 1.0, ts = 0.0;
+        int i = 0;
         if (t < tt[0] || t > tt[K - 1]) {
             if (!c.ice_flat_bc) return set_err(h, FI_ERR_FORCING_RANGE, "TimeInterpolation2D out of range.");
             i = t < tt[0] ? 0 : K - 1;
@@ -1346,14 +1350,20 @@ static int rhs_plain(fi_handle* h, double t, double* u, double* dudt) {
                 ts = t - tt[i];
             }
         }
-        const double* Ha = p.H_tab + (size_t)i * n;
-        const double* Hb = exact ? Ha : Ha + n;
-        kp_ice<<<g, NT, 0, h->stream>>>(Ha, Hb, dti, ts, exact, p.H, n);
-        CKL();
+        Ha = p.H_tab + (size_t)i * n;
+        Hb = exact ? Ha : Ha + n;
     }
     const double rsi = c.rho_seawater / c.rho_ice;
-    kp_haf_ice<<<g, NT, 0, h->stream>>>(p.H, p.z_b, p.z_ss, p.H_af_ref, p.H_af, p.s_i, rsi, c.rho_ice, n);
+    const PlainStage st = stage ? *stage : PlainStage{};
+    kp_head<<<g, NT, 0, h->stream>>>(st, u, nx, ny, c.bc_viscous_border, p.ue, p.z_b_ref, p.u_ref, p.now_u, p.z_b,
+                                     p.s_m, c.rho_uppermantle, Ha, Hb, dti, ts, exact, p.H, p.z_ss, p.H_af_ref, p.H_af,
+                                     p.s_i, rsi, c.rho_ice);
     CKL();
+    const bool maxwell = c.mantle == FI_MANTLE_MAXWELL && c.lithosphere != FI_LITHO_LATERALLY_CONSTANT;
+    if (!maxwell) {
+        kp_copy<<<g, NT, 0, h->stream>>>(u, p.now_u, n);
+        CKL();
+    }
     if (((t - c.t0) / c.dt_sparse_diagnostics) >= (double)h->ctl.count_sparse) {
         if (c.lithosphere == FI_LITHO_RIGID) {
             kp_zero<<<g, NT, 0, h->stream>>>(p.ue, n);
@@ -1402,6 +1412,24 @@ static int rhs_plain(fi_handle* h, double t, double* u, double* dudt) {
         CKL();
         h->ctl.count_sparse += 1;
     }
+    if (maxwell) {
+        // update_dudt!(dudt, u, sim, t, ::MaxwellMantle, ::LaterallyVariableLithosphere)
+        kp_load_moments<<<g, NT, 0, h->stream>>>(p.s_i, p.s_sw, p.s_l, p.s_m, p.mask, p.s_load, p.s_full, p.now_u, u,
+                                                 nx, ny, h->dx, h->dy, p.D, c.litho_poissonratio, p.Mxx, p.Myy, p.Mxy);
+        CKL();
+        kp_div_rows<<<ny, NT, fft64_rows_smem(nx, 1), h->stream>>>(p.s_full, c.g, p.Mxx, p.Myy, p.Mxy, nx, ny, h->dx,
+                                                                   h->dy, p.eta, p.fftrhs, h->d_plans, h->plan_x);
+        CKL();
+        kp_spec_cols<<<nx, NT, fft64_cols_smem(ny, 1), h->stream>>>(p.fftrhs, nx, ny, h->d_spinv, h->d_plans, h->plan_y,
+                                                                    1.0 / ((double)nx * ny));
+        CKL();
+        kp_rows_real<<<ny, NT, fft64_rows_smem(nx, 1), h->stream>>>(p.fftrhs, nx, c.seconds_per_year, p.rhs, h->d_plans,
+                                                                    h->plan_x);
+        CKL();
+        kp_corner_out<<<g, NT, 0, h->stream>>>(p.rhs, nx, ny, c.bc_viscous_border, dudt, p.dudt);
+        CKL();
+        return FI_OK;
+    }
     kp_load_full<<<g, NT, 0, h->stream>>>(p.s_i, p.s_sw, p.s_l, p.s_m, p.mask, p.s_load, p.s_full, n);
     CKL();
     // update_dudt!(dudt, u, sim, t, mantle, lithosphere), src/deformation.jl:21-103
@@ -1438,33 +1466,7 @@ static int rhs_plain(fi_handle* h, double t, double* u, double* dudt) {
         CKL();
         return FI_OK;
     }
-    kp_rhs_init<<<g, NT, 0, h->stream>>>(p.s_full, c.g, p.rhs, n);
-    CKL();
-    kp_dxx<<<g, NT, 0, h->stream>>>(p.bxx, u, nx, ny, h->dx);
-    kp_dyy<<<g, NT, 0, h->stream>>>(p.byy, u, nx, ny, h->dy);
-    kp_dx<<<g, NT, 0, h->stream>>>(p.bx, u, nx, ny, h->dx);
-    kp_dy<<<g, NT, 0, h->stream>>>(p.bxy, p.bx, nx, ny, h->dy);
-    CKL();
-    kp_moments<<<g, NT, 0, h->stream>>>(p.bxx, p.byy, p.bxy, p.D, c.litho_poissonratio, p.Mxx, p.Myy, p.Mxy, n);
-    CKL();
-    kp_dxx<<<g, NT, 0, h->stream>>>(p.bxx, p.Mxx, nx, ny, h->dx);
-    kp_dyy<<<g, NT, 0, h->stream>>>(p.byy, p.Myy, nx, ny, h->dy);
-    kp_dx<<<g, NT, 0, h->stream>>>(p.bx, p.Mxy, nx, ny, h->dx);
-    kp_dy<<<g, NT, 0, h->stream>>>(p.bxy, p.bx, nx, ny, h->dy);
-    CKL();
-    kp_rhs_acc<<<g, NT, 0, h->stream>>>(p.rhs, p.bxx, p.byy, p.bxy, n);
-    kp_fftin<<<g, NT, 0, h->stream>>>(p.rhs, p.eta, p.fftrhs, n);
-    CKL();
-    RET(fft2_64(h, p.fftrhs, nx, ny, 0));
-    kp_spec<<<g, NT, 0, h->stream>>>(p.fftrhs, h->d_spinv, n);
-    CKL();
-    RET(fft2_64(h, p.fftrhs, nx, ny, 1));
-    kp_real_spy<<<g, NT, 0, h->stream>>>(p.fftrhs, c.seconds_per_year, dudt, n);
-    CKL();
-    RET(corner_bc_plain(h, dudt, nx, ny, c.bc_viscous_border));
-    kp_copy<<<g, NT, 0, h->stream>>>(p.dudt, dudt, n);
-    CKL();
-    return FI_OK;
+    return set_err(h, FI_ERR_UNSUPPORTED, "unknown rheology");
 }
 
 static int reduce_host(fi_handle* h, const double* d_partial, int nblk, int stride, double* out) {
@@ -1912,15 +1914,11 @@ static int attempt_plain(fi_handle* h) {
         ct.nsteps_seg += 1;
         return FI_OK;
     }
-    kp_stage<<<gs(n), NT, 0, h->stream>>>(p.tmp, up, dt * A21, k1, n);
-    CKL();
-    RET(rhs_plain(h, t + C2 * dt, p.tmp, p.k2));
-    kp_stage<<<gs(n), NT, 0, h->stream>>>(p.tmp, up, dt * A32, p.k2, n);
-    CKL();
-    RET(rhs_plain(h, t + C3 * dt, p.tmp, p.k3));
-    kp_stage4<<<gs(n), NT, 0, h->stream>>>(un, up, dt, k1, p.k2, p.k3, n);
-    CKL();
-    RET(rhs_plain(h, t + dt, un, k4));
+    const PlainStage s2{1, dt * A21, up, k1, nullptr, nullptr}, s3{1, dt * A32, up, p.k2, nullptr, nullptr},
+        s4{2, dt, up, k1, p.k2, p.k3};
+    RET(rhs_plain(h, t + C2 * dt, p.tmp, p.k2, &s2));
+    RET(rhs_plain(h, t + C3 * dt, p.tmp, p.k3, &s3));
+    RET(rhs_plain(h, t + dt, un, k4, &s4));
     kp_err<<<h->red_blocks, NT, 0, h->stream>>>(up, un, k1, p.k2, p.k3, k4, dt, c.abstol, c.reltol, p.partial, n);
     CKL();
     double s = 0.0;

@@ -1,8 +1,9 @@
-// fi_plain.cu -- the plain FP64 form: one kernel per operation of the reference
-// right-hand side (the broadcast / stencil structure of src/simulation.jl:335-393,
-// src/deformation.jl:91-131 and src/derivatives.jl:48-191), complex 2D FFTs as in
-// the reference's c2c plans, a host-side step controller.  It is the comparison
-// baseline of the fused FP32 form and a second, independent implementation.
+// fi_plain.cu -- the plain FP64 form: the broadcast / stencil structure of the reference
+// right-hand side (src/simulation.jl:335-393, src/deformation.jl:91-131 and
+// src/derivatives.jl:48-191) with complex 2D FFTs as in the reference's c2c plans and a
+// host-side step controller.  The Maxwell path's every-call work runs in six launches;
+// the sparse update and the other rheologies keep one kernel per operation.  It is the
+// comparison baseline of the fused FP32 form and a second, independent implementation.
 #include "fi_device.cuh"
 #include "fi_plain.h"
 
@@ -26,19 +27,6 @@ __global__ void kp_sub_off(double* X, size_t n, const double* off) {
 }
 
 __global__ void kp_copy(double* dst, const double* src, size_t n) { GRID_STRIDE(i, n) dst[i] = src[i]; }
-
-__global__ void kp_bedrock(const double* u, const double* ue, const double* z_b_ref, const double* u_ref,
-                           double* now_u, double* z_b, double* s_m, double rho_um, size_t n) {
-    GRID_STRIDE(i, n) {
-        now_u[i] = u[i];
-        z_b[i] = z_b_ref[i] + ue[i] + u[i];
-        s_m[i] = rho_um * (u[i] - u_ref[i]);
-    }
-}
-
-__global__ void kp_ice(const double* Ha, const double* Hb, double dti, double tt, int exact, double* H, size_t n) {
-    GRID_STRIDE(i, n) H[i] = exact ? Ha[i] : Ha[i] + (Hb[i] - Ha[i]) / dti * tt;
-}
 
 __global__ void kp_haf_ice(const double* H, const double* z_b, const double* z_ss, const double* H_af_ref,
                            double* H_af, double* s_i, double rho_sw_ice, double rho_ice, size_t n) {
@@ -71,6 +59,171 @@ __global__ void kp_load_full(const double* s_i, const double* s_sw, const double
         const double ld = mask[i] * (s_i[i] + s_sw[i] + 0.0);  // the sediment anomaly is zero
         s_load[i] = ld;
         s_full[i] = ld + mask[i] * (s_l[i] + s_m[i]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// One right-hand side of the Maxwell path in six launches.  At the usual sizes a launch costs
+// more than the pass it makes over an L2-resident field, and one kernel per broadcast of the
+// reference took about thirty.  Every product and quotient is rounded where the separate kernels
+// rounded it (__dmul_rn where a following sum would otherwise absorb it), so the results are
+// bitwise theirs.  A coupled 10-yr step at N = 128 (some 25 BS3 attempts): 8567 -> 3027 us.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double corner_off(double c0, double c1, double c2, double c3, double border) {
+    const double s = 0.25 * c0 + 0.25 * c1 + 0.25 * c2 + 0.25 * c3;
+    return s - border;
+}
+
+// the stage vector's value at i: u itself, uprev + a k1, or stage 4 (uprev + dt (a41 k1 + a42 k2 + a43 k3))
+__device__ __forceinline__ double stage_value(const PlainStage& st, const double* u, size_t i) {
+    if (st.kind == 0) return u[i];
+    if (st.kind == 1) return st.up[i] + st.a * st.k1[i];
+    return st.up[i] + st.a * (A41 * st.k1[i] + A42 * st.k2[i] + A43 * st.k3[i]);
+}
+
+// stage vector, its corner BC, bedrock, ice, height above floatation and their anomalies.  u is
+// only read (its corners by every block); now_u gets the corrected vector.
+__global__ void kp_head(PlainStage st, const double* u, int nx, int ny, double border, const double* ue,
+                        const double* z_b_ref, const double* u_ref, double* now_u, double* z_b, double* s_m,
+                        double rho_um, const double* Ha, const double* Hb, double dti, double tt, int exact, double* H,
+                        const double* z_ss, const double* H_af_ref, double* H_af, double* s_i, double rho_sw_ice,
+                        double rho_ice) {
+    const size_t n = (size_t)nx * ny;
+    const double off = corner_off(stage_value(st, u, 0), stage_value(st, u, nx - 1), stage_value(st, u, n - nx),
+                                  stage_value(st, u, n - 1), border);
+    GRID_STRIDE(i, n) {
+        const double uv = stage_value(st, u, i) - off;
+        now_u[i] = uv;
+        const double zb = z_b_ref[i] + ue[i] + uv;
+        z_b[i] = zb;
+        s_m[i] = rho_um * (uv - u_ref[i]);
+        double h;
+        if (Ha) {
+            h = exact ? Ha[i] : Ha[i] + (Hb[i] - Ha[i]) / dti * tt;
+            H[i] = h;
+        } else {
+            h = H[i];
+        }
+        double m = zb - z_ss[i];
+        if (m > 0) m = 0;
+        double v = h + m * rho_sw_ice;
+        v = v > 0 ? v : 0.0;
+        H_af[i] = v;
+        s_i[i] = rho_ice * (v - H_af_ref[i]);
+    }
+}
+
+// d/dx along row r (one-sided at the ends)
+__device__ __forceinline__ double dx_at(const double* r, int i, int nx, double Dx) {
+    if (i == 0) return (r[1] - r[0]) / Dx;
+    if (i == nx - 1) return (r[nx - 1] - r[nx - 2]) / Dx;
+    return (r[i + 1] - r[i - 1]) / (2 * Dx);
+}
+__device__ __forceinline__ double dxx_at(const double* r, int i, int nx, double Dx) {
+    const int c = i < 1 ? 1 : (i > nx - 2 ? nx - 2 : i);
+    return (r[c + 1] - 2 * r[c] + r[c - 1]) / (Dx * Dx);
+}
+__device__ __forceinline__ double dyy_at(const double* u, int i, int j, int nx, int ny, double Dy) {
+    const size_t e = (size_t)j * nx + i;
+    if (j > 0 && j < ny - 1) return (u[e + nx] - 2 * u[e] + u[e - nx]) / (Dy * Dy);
+    if (j == 0) return (u[e + 2 * (size_t)nx] - 2 * u[e + nx] + u[e]) / (Dy * Dy);
+    return (u[e] - 2 * u[e - nx] + u[e - 2 * (size_t)nx]) / (Dy * Dy);
+}
+// d/dy of d/dx
+__device__ __forceinline__ double dxy_at(const double* u, int i, int j, int nx, int ny, double Dx, double Dy) {
+    const double* r = u + (size_t)j * nx;
+    if (j == 0) return (dx_at(r + nx, i, nx, Dx) - dx_at(r, i, nx, Dx)) / Dy;
+    if (j == ny - 1) return (dx_at(r, i, nx, Dx) - dx_at(r - nx, i, nx, Dx)) / Dy;
+    return (dx_at(r + nx, i, nx, Dx) - dx_at(r - nx, i, nx, Dx)) / (2 * Dy);
+}
+
+// column anomalies, bending moments of now_u; u <- now_u (the BC's in-place change)
+__global__ void kp_load_moments(const double* s_i, const double* s_sw, const double* s_l, const double* s_m,
+                                const double* mask, double* s_load, double* s_full, const double* now_u, double* u,
+                                int nx, int ny, double Dx, double Dy, const double* D, double nu, double* Mxx,
+                                double* Myy, double* Mxy) {
+    GRID_STRIDE(e, (size_t)nx * ny) {
+        const int i = (int)(e % nx), j = (int)(e / nx);
+        const double ld = __dmul_rn(mask[e], s_i[e] + s_sw[e] + 0.0);
+        s_load[e] = ld;
+        s_full[e] = ld + mask[e] * (s_l[e] + s_m[e]);
+        const double bxx = dxx_at(now_u + (e - i), i, nx, Dx), byy = dyy_at(now_u, i, j, nx, ny, Dy);
+        const double bxy = dxy_at(now_u, i, j, nx, ny, Dx, Dy);
+        Mxx[e] = -D[e] * (nu * byy + bxx);
+        Myy[e] = -D[e] * (nu * bxx + byy);
+        Mxy[e] = -D[e] * (1 - nu) * bxy;
+        u[e] = now_u[e];
+    }
+}
+
+// a row of rhs = -g s_full + Mxx_xx + 2 Mxy_xy + Myy_yy, times K/(2 eta), and its row transform
+__global__ void __launch_bounds__(256)
+kp_div_rows(const double* s_full, double g, const double* Mxx, const double* Myy, const double* Mxy, int nx, int ny,
+            double Dx, double Dy, const double* eta, double2* f, const FftPlan* plans, int plan) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ FftPlan s_plan;
+    const int j = blockIdx.x;
+    if (threadIdx.x == 0) s_plan = plans[plan];
+    double2* b0 = (double2*)smem;
+    double2* b1 = b0 + nx;
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+        const size_t e = (size_t)j * nx + i;
+        const double bxx = dxx_at(Mxx + (size_t)j * nx, i, nx, Dx), byy = dyy_at(Myy, i, j, nx, ny, Dy);
+        const double bxy = dxy_at(Mxy, i, j, nx, ny, Dx, Dy);
+        const double rhs = __dmul_rn(-g, s_full[e]) + (bxx + (2 * bxy + byy));
+        b0[i] = make_double2(rhs * 1.0 / (2 * eta[e]), 0.0);
+    }
+    __syncthreads();
+    double2* r = fft_batch<false, double>(b0, b1, s_plan, 1, nx);
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) f[(size_t)j * nx + i] = r[i];
+}
+
+// a column: transform, times 1/(R |k|), inverse transform with its scale
+__global__ void __launch_bounds__(256)
+kp_spec_cols(double2* f, int nx, int ny, const double* spinv, const FftPlan* plans, int plan, double scale) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ FftPlan s_plan;
+    const int kx = blockIdx.x;
+    if (threadIdx.x == 0) s_plan = plans[plan];
+    double2* b0 = (double2*)smem;
+    double2* b1 = b0 + ny;
+    for (int y = threadIdx.x; y < ny; y += blockDim.x) b0[y] = f[(size_t)y * nx + kx];
+    __syncthreads();
+    double2* r = fft_batch<false, double>(b0, b1, s_plan, 1, ny);
+    double2* o = r == b0 ? b1 : b0;
+    for (int y = threadIdx.x; y < ny; y += blockDim.x) {
+        const double s = spinv[(size_t)y * nx + kx];
+        r[y] = make_double2(r[y].x * s, r[y].y * s);
+    }
+    __syncthreads();
+    double2* q = fft_batch<true, double>(r, o, s_plan, 1, ny);
+    for (int y = threadIdx.x; y < ny; y += blockDim.x)
+        f[(size_t)y * nx + kx] = make_double2(q[y].x * scale, q[y].y * scale);
+}
+
+// inverse row transform, real part times the seconds of a year
+__global__ void __launch_bounds__(256)
+kp_rows_real(const double2* f, int nx, double spy, double* raw, const FftPlan* plans, int plan) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ FftPlan s_plan;
+    if (threadIdx.x == 0) s_plan = plans[plan];
+    double2* b0 = (double2*)smem;
+    double2* b1 = b0 + nx;
+    const size_t r0 = (size_t)blockIdx.x * nx;
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) b0[i] = f[r0 + i];
+    __syncthreads();
+    double2* r = fft_batch<true, double>(b0, b1, s_plan, 1, nx);
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) raw[r0 + i] = r[i].x * spy;
+}
+
+// corner BC of raw into dudt and its copy
+__global__ void kp_corner_out(const double* raw, int nx, int ny, double border, double* dudt, double* now_dudt) {
+    const size_t n = (size_t)nx * ny;
+    const double off = corner_off(raw[0], raw[nx - 1], raw[n - nx], raw[n - 1], border);
+    GRID_STRIDE(i, n) {
+        const double v = raw[i] - off;
+        dudt[i] = v;
+        now_dudt[i] = v;
     }
 }
 
@@ -109,80 +262,6 @@ __global__ void kp_sealevel(const double* H, const double* H_af, const double* z
     }
 }
 
-__global__ void kp_rhs_init(const double* s_full, double g, double* rhs, size_t n) {
-    GRID_STRIDE(i, n) rhs[i] = -g * s_full[i];
-}
-
-__global__ void kp_dxx(double* du, const double* u, int nx, int ny, double Dx) {
-    GRID_STRIDE(e, (size_t)nx * ny) {
-        const int i = (int)(e % nx);
-        const size_t r = e - i;
-        const int c = i < 1 ? 1 : (i > nx - 2 ? nx - 2 : i);
-        du[e] = (u[r + c + 1] - 2 * u[r + c] + u[r + c - 1]) / (Dx * Dx);
-    }
-}
-
-__global__ void kp_dyy(double* du, const double* u, int nx, int ny, double Dy) {
-    GRID_STRIDE(e, (size_t)nx * ny) {
-        const int i = (int)(e % nx), j = (int)(e / nx);
-        const int c = j < 1 ? 1 : (j > ny - 2 ? ny - 2 : j);
-        if (j > 0 && j < ny - 1)
-            du[e] = (u[(size_t)(c + 1) * nx + i] - 2 * u[(size_t)c * nx + i] + u[(size_t)(c - 1) * nx + i]) / (Dy * Dy);
-        else if (j == 0)
-            du[e] = (u[(size_t)2 * nx + i] - 2 * u[(size_t)nx + i] + u[i]) / (Dy * Dy);
-        else
-            du[e] = (u[(size_t)(ny - 1) * nx + i] - 2 * u[(size_t)(ny - 2) * nx + i] + u[(size_t)(ny - 3) * nx + i]) /
-                    (Dy * Dy);
-    }
-}
-
-__global__ void kp_dx(double* du, const double* u, int nx, int ny, double Dx) {
-    GRID_STRIDE(e, (size_t)nx * ny) {
-        const int i = (int)(e % nx);
-        if (i == 0) du[e] = (u[e + 1] - u[e]) / Dx;
-        else if (i == nx - 1) du[e] = (u[e] - u[e - 1]) / Dx;
-        else du[e] = (u[e + 1] - u[e - 1]) / (2 * Dx);
-    }
-}
-
-__global__ void kp_dy(double* du, const double* u, int nx, int ny, double Dy) {
-    GRID_STRIDE(e, (size_t)nx * ny) {
-        const int j = (int)(e / nx);
-        if (j == 0) du[e] = (u[e + nx] - u[e]) / Dy;
-        else if (j == ny - 1) du[e] = (u[e] - u[e - nx]) / Dy;
-        else du[e] = (u[e + nx] - u[e - nx]) / (2 * Dy);
-    }
-}
-
-__global__ void kp_moments(const double* bxx, const double* byy, const double* bxy, const double* D, double nu,
-                           double* Mxx, double* Myy, double* Mxy, size_t n) {
-    GRID_STRIDE(i, n) {
-        Mxx[i] = -D[i] * (nu * byy[i] + bxx[i]);
-        Myy[i] = -D[i] * (nu * bxx[i] + byy[i]);
-        Mxy[i] = -D[i] * (1 - nu) * bxy[i];
-    }
-}
-
-__global__ void kp_rhs_acc(double* rhs, const double* bxx, const double* byy, const double* bxy, size_t n) {
-    GRID_STRIDE(i, n) rhs[i] += bxx[i] + (2 * bxy[i] + byy[i]);
-}
-
-__global__ void kp_fftin(const double* rhs, const double* eta, double2* f, size_t n) {
-    GRID_STRIDE(i, n) f[i] = make_double2(rhs[i] * 1.0 / (2 * eta[i]), 0.0);
-}
-
-__global__ void kp_spec(double2* f, const double* spinv, size_t n) {
-    GRID_STRIDE(i, n) {
-        const double s = spinv[i];
-        f[i].x *= s;
-        f[i].y *= s;
-    }
-}
-
-__global__ void kp_real_spy(const double2* f, double spy, double* dudt, size_t n) {
-    GRID_STRIDE(i, n) dudt[i] = f[i].x * spy;
-}
-
 __global__ void kp_cmul(double2* P, const double2* G, size_t n) {
     GRID_STRIDE(i, n) {
         const double2 a = P[i], b = G[i];
@@ -209,11 +288,6 @@ __global__ void kp_zero(double* X, size_t n) { GRID_STRIDE(i, n) X[i] = 0.0; }
 // integrator helpers (perform_step!(integrator, ::BS3Cache))
 __global__ void kp_stage(double* out, const double* uprev, double a, const double* k, size_t n) {
     GRID_STRIDE(i, n) out[i] = uprev[i] + a * k[i];
-}
-
-__global__ void kp_stage4(double* out, const double* uprev, double dt, const double* k1, const double* k2,
-                          const double* k3, size_t n) {
-    GRID_STRIDE(i, n) out[i] = uprev[i] + dt * (A41 * k1[i] + A42 * k2[i] + A43 * k3[i]);
 }
 
 __global__ void kp_err(const double* uprev, const double* u, const double* k1, const double* k2, const double* k3,
