@@ -187,24 +187,6 @@ struct EpiIdftY {
     __device__ __forceinline__ void row_done(int, int) const {}
 };
 
-// row (b, p), col c -> out[b][c][p] in FP32, stored or accumulated
-struct EpiNchw {
-    float* out;
-    int S2, accumulate;
-    __device__ __forceinline__ void operator()(int, int row, int c0, const float* v, int) const {
-        const int b = row / S2, p = row - b * S2;
-        float* o = out + ((size_t)b * C + c0) * S2 + p;
-        if (accumulate) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) o[(size_t)i * S2] += v[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 16; i++) o[(size_t)i * S2] = v[i];
-        }
-    }
-    __device__ __forceinline__ void row_done(int, int) const {}
-};
-
 // inverse DFT along x + pointwise path + bias: batch z = (b, y), row x, col c.  Saves z
 // (FP32) and writes the activation, both NCHW.
 struct EpiPixAct {
@@ -227,15 +209,21 @@ struct EpiPixAct {
     __device__ __forceinline__ void row_done(int, int) const {}
 };
 
-// batch z = (b, y), row x, col c -> out[b][c][y*S + x] (FP32)
-struct EpiPixStore {
-    float* out;
+// gradient of a layer's input, batch z = (b, y), row x, col c, times GELU'(zs) of the layer below
+// (identity when zs is null) -> dz[b][c][y*S + x] in BF16.  dz may be the operand that the product
+// read: a tile's pixels are read by that tile alone, before its epilogue.
+struct EpiPixBwd {
+    const float* zs;
+    bf16* dz;
     int S, S2;
     __device__ __forceinline__ void operator()(int z, int x, int c0, const float* v, int) const {
         const int b = z / S, y = z - b * S;
-        float* o = out + ((size_t)b * C + c0) * S2 + (size_t)y * S + x;
+        const size_t o = ((size_t)b * C + c0) * S2 + (size_t)y * S + x;
+        float zv[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) o[(size_t)i * S2] = v[i];
+        for (int i = 0; i < 16; i++) zv[i] = zs ? zs[o + (size_t)i * S2] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) dz[o + (size_t)i * S2] = __float2bfloat16_rn(zs ? v[i] * gelu_grad(zv[i]) : v[i]);
     }
     __device__ __forceinline__ void row_done(int, int) const {}
 };
@@ -255,33 +243,305 @@ struct EpiProj {
     __device__ __forceinline__ void row_done(int z, int p) { q[(size_t)z * S2 + p] = acc + b2[0]; }
 };
 
-// projection adjoint (recomputes the hidden pre-activation a; batch z = b, row p):
-// da = dq Q2 GELU'(a) in [(b,p)][j] and [b][j][p], the hidden GELU(a) in [b][128 + j][p]
-struct EpiProjBwd {
-    const float* b1;
-    const float* Q2;
-    const float* dq;
-    bf16* da_rows;
-    bf16* daT;
-    int S2;
-    __device__ __forceinline__ void operator()(int b, int p, int j0, const float* v, int) const {
-        const size_t row = (size_t)b * S2 + p;
-        const float g = dq[row];
-        float d[16];
-        bf16* t = daT + ((size_t)b * 2 * PW + j0) * S2 + p;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float a = v[i] + b1[j0 + i];
-            float ga, gpa;
-            gelu_both(a, ga, gpa);
-            d[i] = g * Q2[j0 + i] * gpa;
-            t[(size_t)i * S2] = __float2bfloat16_rn(d[i]);
-            t[(size_t)(PW + i) * S2] = __float2bfloat16_rn(ga);
+// ---------------------------------------------------------------------------
+// weight gradients of the pointwise layers: slices of SLICE pixels
+// ---------------------------------------------------------------------------
+constexpr int SLICE = 512;  // pixels per split-K slice (S2 is a multiple of 1024)
+
+// part[slice][32][NR] = sum over the slice's pixels of dz[32][p] x act[NR][p], one 128 x N tensor-core
+// tile whose rows beyond 32 (and columns beyond NR) hold whatever the operand buffers overlap: only
+// their own, unread, results depend on it.  A slice is one copy of (32 + NR) KB, 32 MMAs and one
+// wait; three blocks an SM keep copies and MMAs of different slices in flight.  As a general
+// product in eight chunks of K, each with a copy, a wait and two block barriers, it took 38 us at
+// 32 samples of 128 x 128 (67 MB read), this one 31 us.
+template <int NR>
+__global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ dz, const bf16* __restrict__ act,
+                                               long long act_s, int S2, int nslices, float* part, int* err,
+                                               long long polls) {
+    constexpr int NG = (NR + 7) / 8, N = (NR + 15) / 16 * 16, KG = SLICE / 8;
+    constexpr int A_LBO = 4 * 128, B_LBO = NG * 128, A_BYTES = KG * A_LBO;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ns = S2 / SLICE;
+    const uint32_t sa = tc_smem_u32(smem), sb = sa + A_BYTES;
+    // a piece is 8 pixels (16 bytes) of a row r, to row r % 8 of core matrix (pixel group g, r / 8);
+    // eight neighbouring threads take eight rows of one core matrix (contiguous in shared memory),
+    // the next eight the next pixel group (contiguous in global memory)
+    auto stage = [&](int z) {
+        const int b = z / ns;
+        const size_t px = (size_t)(z - b * ns) * SLICE;
+        const bf16* pa = dz + (size_t)b * C * S2 + px;
+        const bf16* pb = act + (size_t)b * act_s + px;
+        for (int v = tid; v < (4 + NG) * 8 * KG; v += 256) {
+            const int rl = v & 7, g = (v >> 3) % KG, rg = v / (8 * KG);
+            if (rg < 4)
+                cp_async16(sa + g * A_LBO + rg * 128 + rl * 16, pa + (size_t)(rg * 8 + rl) * S2 + 8 * g, true);
+            else if ((rg - 4) * 8 + rl < NR)
+                cp_async16(sb + g * B_LBO + (rg - 4) * 128 + rl * 16, pb + (size_t)((rg - 4) * 8 + rl) * S2 + 8 * g,
+                           true);
         }
-        store16(da_rows + (size_t)row * PW + j0, d);
+        cp_async_commit();
+    };
+    int z = blockIdx.x;
+    if (z < nslices) stage(z);
+    if (warp == 0) {
+        tc_alloc(&tmem_base, 64);
+        tc_relinquish();
     }
-    __device__ __forceinline__ void row_done(int, int) const {}
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_fail = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    int n = 0;  // slices committed
+    for (; z < nslices; z += gridDim.x) {
+        cp_async_wait<0>();
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            for (int ks = 0; ks < SLICE / 16; ks++)
+                tc_mma(tmem, tc_smem_desc(sa + 2 * ks * A_LBO, A_LBO, 128), tc_smem_desc(sb + 2 * ks * B_LBO, B_LBO, 128),
+                       tc_instr_desc(TC_BM, N), ks > 0);
+            tc_commit(&bar);
+            if (!mbar_wait(&bar, (uint32_t)(n & 1), polls)) s_fail = 1;
+        }
+        n++;
+        __syncthreads();
+        if (s_fail) break;
+        tc_fence_after();
+        if (z + (int)gridDim.x < nslices) stage(z + gridDim.x);
+        if (warp == 0) {
+            float* o = part + ((size_t)z * C + lane) * NR;
+#pragma unroll
+            for (int c0 = 0; c0 < N; c0 += 16) {
+                float v[16];
+                tc_ld16(tmem + c0, v);
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    if (c0 + i < NR) o[c0 + i] = v[i];
+            }
+            tc_fence_before();
+        }
+        // the next slice's MMAs are issued after the next __syncthreads()
+    }
+    cp_async_wait<0>();
+    if (s_fail && tid == 0) {
+        if (err) atomicExch(err, FI_ERR_TIMEOUT);
+        mbar_wait(&bar, (uint32_t)((n - 1) & 1));  // let the issued MMAs finish before their memory goes
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc_dealloc(tmem, 64);
+}
+template <int NR>
+constexpr int wgrad_smem() { return SLICE / 8 * (4 + (NR + 7) / 8) * 128 + 1024; }
+
+// ---------------------------------------------------------------------------
+// adjoint of the projection, fused: per slice of SLICE pixels, in tiles of 128 pixels,
+//   a = v Q1^T + b1 (recomputed), da = dq Q2 GELU'(a), h = GELU(a)
+//   dz = da Q1 (gradient of the last layer's output, BF16 NCHW)
+//   part[slice][j][c] = sum da_j v_c (c < 32), sum da_j (c = 32), sum h_j dq (c = 33)
+// da and h exist only as BF16 tiles in shared memory: 16-byte pieces of 8 hidden units of a pixel,
+// which serve as the pixels x units operand of dz and, transposed by the descriptors, as the
+// units x pixels operand of the weight gradients; likewise the tile of v (channels 0..33) for a
+// and for the weight gradients.  Three products of separate kernels moved 1.2 GB of da and h at
+// 32 samples of 128 x 128; what is left is bound by the instructions of erff and expf.
+// 434 us in four kernels -> 159 us (103 M instructions).
+// ---------------------------------------------------------------------------
+struct ProjBwdArgs {
+    const bf16* v;       // last activation buffer [b][VC][S2]
+    const bf16 *Q1, *Q1T;  // [128][32], [32][128]
+    const float *b1, *Q2, *dq;
+    bf16* dz;
+    float* part;
+    int S2, nslices;
+    int* err;
+    long long polls;
 };
+constexpr int PB_V = 6 * 2048, PB_V_OFF = 0, PB_Q1 = 2 * PB_V, PB_Q1T = PB_Q1 + 8192, PB_DA = PB_Q1T + 8192,
+              PB_H = PB_DA + 32768, PB_W = PB_H + 32768, PB_SMEM = PB_W + 1024;
+
+__global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ ProjBwdArgs g) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ uint32_t tmem_base;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S2 = g.S2, ns = S2 / SLICE;
+    const uint32_t s0 = tc_smem_u32(smem);
+    float* const sb1 = (float*)(smem + PB_W);
+    float* const sQ2 = sb1 + PW;
+    // tile t of this block's sequence (4 per slice): pixels of sample b from px
+    auto where = [&](int t, int& b, size_t& px) {
+        const int z = blockIdx.x + (t >> 2) * gridDim.x;
+        b = z / ns;
+        px = (size_t)(z - b * ns) * SLICE + (t & 3) * 128;
+    };
+    auto stage = [&](int t) {
+        int b;
+        size_t px;
+        where(t, b, px);
+        const bf16* p = g.v + (size_t)b * VC * S2 + px;
+        const uint32_t d = s0 + PB_V_OFF + (t & 1) * PB_V;
+        // 16-byte piece: 8 pixels of channel c; eight neighbouring threads take eight channels of one
+        // core matrix
+        for (int v = tid; v < (VC + 7) / 8 * 128; v += 256) {
+            const int c = (v >> 7) * 8 + (v & 7), q = (v >> 3) & 15;
+            if (c < VC) cp_async16(d + (c >> 3) * 2048 + q * 128 + (c & 7) * 16, p + (size_t)c * S2 + 8 * q, true);
+        }
+        cp_async_commit();
+    };
+    const int my = g.nslices > (int)blockIdx.x ? (g.nslices - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    const int ntiles = 4 * my;
+    for (int v = tid; v < PW * 4; v += 256) {
+        const int r = v >> 2, q = v & 3;
+        cp_async16(s0 + PB_Q1 + q * (PW * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1 + r * C + 8 * q, true);
+    }
+    for (int v = tid; v < C * 16; v += 256) {
+        const int r = v >> 4, q = v & 15;
+        cp_async16(s0 + PB_Q1T + q * (C * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1T + r * PW + 8 * q, true);
+    }
+    if (tid < PW) {
+        sb1[tid] = g.b1[tid];
+        sQ2[tid] = g.Q2[tid];
+    }
+    if (ntiles > 0) stage(0);
+    if (warp == 0) {
+        tc_alloc(&tmem_base, 256);
+        tc_relinquish();
+    }
+    if (tid == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_fail = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base, tW1 = tmem + PW, tW2 = tmem + PW + 48;
+    const int quad = warp & 3, half = warp >> 2, pr = quad * 32 + lane;  // pixel row of the tile, column half
+    const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+    int stage_bar = -1;  // thread 0: the barrier of its last commit (0, 1), and the phase
+    uint32_t last_phase = 0;
+    for (int t = 0; t < ntiles; t++) {
+        const uint32_t ph = (uint32_t)(t & 1);
+        const uint32_t sv = s0 + PB_V_OFF + (t & 1) * PB_V;
+        cp_async_wait<0>();
+        fence_async_smem();
+        __syncthreads();
+        // hidden layer: pixels (MN-major v, 32 channels) x units
+        if (tid == 0) {
+            tc_fence_after();
+            for (int ks = 0; ks < 2; ks++)
+                tc_mma(tmem, tc_smem_desc(sv + 2 * ks * 2048, 2048, 128),
+                       tc_smem_desc(s0 + PB_Q1 + 2 * ks * (PW * 16), PW * 16, 128),
+                       tc_instr_desc(TC_BM, PW) | (1u << 15), ks > 0);
+            tc_commit(&bars[0]);
+            stage_bar = 0;
+            last_phase = ph;
+        }
+        // the other tile buffer was last read by the previous tile's products, which are done
+        if (t + 1 < ntiles) stage(t + 1);
+        int b;
+        size_t px;
+        where(t, b, px);
+        const float gq = g.dq[(size_t)b * S2 + px + pr];
+        if (tid == 0 && !mbar_wait(&bars[0], ph, g.polls)) s_fail = 1;
+        __syncthreads();
+        if (s_fail) break;
+        tc_fence_after();
+        // da and h of this thread's pixel, 64 units
+        unsigned char* const dda = smem + PB_DA + (pr >> 3) * 2048 + (pr & 7) * 16;
+#pragma unroll 1
+        for (int j0 = half * 64; j0 < half * 64 + 64; j0 += 16) {
+            float v[16], h[16];
+            tc_ld16(tmem + lanes + (uint32_t)j0, v);
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                float ga, gpa;
+                gelu_both(v[i] + sb1[j0 + i], ga, gpa);
+                v[i] = gq * sQ2[j0 + i] * gpa;
+                h[i] = ga;
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const float *a = v + 8 * q, *c = h + 8 * q;
+                *(uint4*)(dda + ((j0 >> 3) + q) * 128) =
+                    make_uint4(pack2(a[0], a[1]), pack2(a[2], a[3]), pack2(a[4], a[5]), pack2(a[6], a[7]));
+                *(uint4*)(dda + (PB_H - PB_DA) + ((j0 >> 3) + q) * 128) =
+                    make_uint4(pack2(c[0], c[1]), pack2(c[2], c[3]), pack2(c[4], c[5]), pack2(c[6], c[7]));
+            }
+        }
+        tc_fence_before();
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            const uint32_t da = s0 + PB_DA, hh = s0 + PB_H;
+            // dz: pixels x units (K) times Q1T; the hidden accumulator's first columns are free again
+            for (int ks = 0; ks < PW / 16; ks++)
+                tc_mma(tmem, tc_smem_desc(da + 2 * ks * 128, 128, 2048),
+                       tc_smem_desc(s0 + PB_Q1T + 2 * ks * (C * 16), C * 16, 128), tc_instr_desc(TC_BM, C), ks > 0);
+            // weight gradients: units (MN-major) x pixels (K) times channels
+            for (int ks = 0; ks < 8; ks++) {
+                const uint32_t acc = (t & 3) > 0 || ks > 0;
+                tc_mma(tW1, tc_smem_desc(da + 2 * ks * 2048, 2048, 128), tc_smem_desc(sv + 2 * ks * 128, 128, 2048),
+                       tc_instr_desc(TC_BM, 48) | (1u << 15), acc);
+                tc_mma(tW2, tc_smem_desc(hh + 2 * ks * 2048, 2048, 128),
+                       tc_smem_desc(sv + 4 * 2048 + 2 * ks * 128, 128, 2048), tc_instr_desc(TC_BM, 16) | (1u << 15), acc);
+            }
+            tc_commit(&bars[1]);
+            stage_bar = 1;
+            last_phase = ph;
+            if (!mbar_wait(&bars[1], ph, g.polls)) s_fail = 1;
+        }
+        __syncthreads();
+        if (s_fail) break;
+        tc_fence_after();
+        {
+            float v[16];
+            tc_ld16(tmem + lanes + (uint32_t)(half * 16), v);
+            bf16* o = g.dz + ((size_t)b * C + half * 16) * S2 + px + pr;
+#pragma unroll
+            for (int i = 0; i < 16; i++) o[(size_t)i * S2] = __float2bfloat16_rn(v[i]);
+        }
+        if ((t & 3) == 3) {
+            const int z = blockIdx.x + (t >> 2) * gridDim.x;
+            float* o = g.part + ((size_t)z * PW + pr) * VC;
+            float v[16];
+            if (half == 0) {
+#pragma unroll
+                for (int c0 = 0; c0 < 32; c0 += 16) {
+                    tc_ld16(tW1 + lanes + (uint32_t)c0, v);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) o[c0 + i] = v[i];
+                }
+            } else {
+                tc_ld16(tW1 + lanes + 32u, v);
+                o[C] = v[0];
+                tc_ld16(tW2 + lanes, v);
+                o[C + 1] = v[1];
+            }
+        }
+        tc_fence_before();
+        // the next tile's MMAs are issued after the next __syncthreads()
+    }
+    cp_async_wait<0>();
+    if (s_fail && tid == 0) {
+        if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
+        if (stage_bar >= 0) mbar_wait(&bars[stage_bar], last_phase);  // let the issued MMAs finish
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc_dealloc(tmem, 256);
+}
 
 // ---------------------------------------------------------------------------
 // element-wise and reduction kernels
@@ -305,29 +565,6 @@ __global__ void k_fill_channel(bf16* v, int B, int S2, int ch, float value) {
     if (i >= (size_t)B * S2) return;
     const int b = (int)(i / S2), p = (int)(i - (size_t)b * S2);
     v[((size_t)b * VC + ch) * S2 + p] = __float2bfloat16_rn(value);
-}
-
-// dz = dv * GELU'(z) (identity when z is null) -> BF16 NCHW and, if dzh, NHWC.
-// One block per (sample, 64 pixels).
-__global__ void __launch_bounds__(256) k_act_bwd(const float* __restrict__ dv, const float* __restrict__ z,
-                                                 bf16* dz, bf16* dzh, int S2) {
-    __shared__ float tile[C][65];
-    const int tiles = S2 / 64;
-    const int b = blockIdx.x / tiles, p0 = (blockIdx.x - b * tiles) * 64;
-    for (int i = threadIdx.x; i < C * 64; i += 256) {
-        const int c = i >> 6, px = i & 63;
-        const size_t idx = ((size_t)b * C + c) * S2 + p0 + px;
-        float d = dv[idx];
-        if (z) d *= gelu_grad(z[idx]);
-        dz[idx] = __float2bfloat16_rn(d);
-        tile[c][px] = d;
-    }
-    if (!dzh) return;
-    __syncthreads();
-    for (int i = threadIdx.x; i < 64 * C; i += 256) {
-        const int px = i >> 5, c = i & 31;
-        dzh[((size_t)b * S2 + p0 + px) * C + c] = __float2bfloat16_rn(tile[c][px]);
-    }
 }
 
 // loss gradient: weighted MSE against target, loss = (1/n) sum_i w_b(i) (q_i - t_i)^2 with
@@ -431,39 +668,35 @@ __global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* __restrict__ Z, 
     }
 }
 
-// split-K partials [z][MN] summed over z and added to grad[base + map[i]] (map < 0: not a
-// parameter; grad is zeroed before the backward pass; map is one-to-one), in two passes
-// with a fixed summation order, so that gradients are the same on every run.  Pass 1:
-// block (x, y) sums the z range y of gridDim.y for 256 consecutive i and leaves the sum
-// in row z0 of its own range.  Pass 2 (k_reduce_map_fin) adds the ranges in order.
-__global__ void k_reduce_map(float* part, int nz, int MN, const int* __restrict__ map) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= MN) return;
-    if (map[i] < 0) return;
-    const int per = (nz + gridDim.y - 1) / gridDim.y, z0 = blockIdx.y * per, z1 = min(nz, z0 + per);
-    if (z1 <= z0) return;
-    float s = 0.f;
-    for (int z = z0; z < z1; z++) s += part[(size_t)z * MN + i];
-    part[(size_t)z0 * MN + i] = s;
+// split-K partials [z][MN] summed over z and added to grad[base + map[i]] (grad is zeroed before the
+// backward pass; map is one-to-one), in a fixed order, so that gradients are the same on every run:
+// each of at most 64 ranges of `per` consecutive z in order (range y and y + 32 by row y of the
+// block), then the ranges in order.
+__global__ void __launch_bounds__(1024) k_reduce_map(const float* __restrict__ part, int nz, int MN, int per,
+                                                     const int* __restrict__ map, float* grad, long long base) {
+    __shared__ float sm[64][33];
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    for (int y = threadIdx.y; y < 64; y += 32) {
+        float s = 0.f;
+        if (i < MN) {
+            const int z1 = min(nz, (y + 1) * per);
+#pragma unroll 8
+            for (int z = y * per; z < z1; z++) s += part[(size_t)z * MN + i];
+        }
+        sm[y][threadIdx.x] = s;
+    }
+    __syncthreads();
+    if (threadIdx.y == 0 && i < MN) {
+        float a = 0.f;
+        for (int y = 0; y * per < nz; y++) a += sm[y][threadIdx.x];
+        grad[base + map[i]] += a;
+    }
 }
 
-__global__ void k_reduce_map_fin(const float* __restrict__ part, int nz, int MN, int ny,
-                                 const int* __restrict__ map, float* grad, long long base) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= MN) return;
-    const int t = map[i];
-    if (t < 0) return;
-    const int per = (nz + ny - 1) / ny;
-    float s = 0.f;
-    for (int z0 = 0; z0 < nz; z0 += per) s += part[(size_t)z0 * MN + i];
-    grad[base + t] += s;
-}
-
-static cudaError_t reduce_map(float* part, cudaStream_t st, int nz, int MN, int ny, const int* map, float* grad,
-                              long long base) {
-    const unsigned gx = (unsigned)((MN + 255) / 256);
-    k_reduce_map<<<dim3(gx, ny), 256, 0, st>>>(part, nz, MN, map);
-    k_reduce_map_fin<<<gx, 256, 0, st>>>(part, nz, MN, ny, map, grad, base);
+// ranges: at most this many (<= 64)
+static cudaError_t reduce_map(const float* part, cudaStream_t st, int nz, int MN, int ranges, const int* map,
+                              float* grad, long long base) {
+    k_reduce_map<<<(MN + 31) / 32, dim3(32, 32), 0, st>>>(part, nz, MN, (nz + ranges - 1) / ranges, map, grad, base);
     return cudaGetLastError();
 }
 
@@ -531,7 +764,7 @@ using namespace fi;
 using namespace fi::fno;
 
 struct fi_fno {
-    int S = 0, S2 = 0, maxB = 0, device = 0, SL = 0, ns = 0;
+    int S = 0, S2 = 0, maxB = 0, device = 0, ns = 0;
     Offsets o{};
     cudaStream_t st = nullptr;
     float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
@@ -544,9 +777,10 @@ struct fi_fno {
          *G2T = nullptr, *G1T = nullptr;
     // activations (saved for the backward pass) and scratch
     bf16 *xe = nullptr, *vext[NLAYER + 1] = {}, *Tb = nullptr, *Zm[NLAYER] = {}, *Yb = nullptr, *Gt = nullptr,
-         *dz = nullptr, *dYm = nullptr, *da_rows = nullptr, *daT = nullptr;
-    float *zs[NLAYER] = {}, *q = nullptr, *dq = nullptr, *dvf = nullptr, *part = nullptr, *scal = nullptr;
+         *dz = nullptr, *dYm = nullptr;
+    float *zs[NLAYER] = {}, *q = nullptr, *dq = nullptr, *part = nullptr, *scal = nullptr;
     int *map_loc = nullptr, *map_proj = nullptr, *map_lift = nullptr, *err = nullptr;
+    int nsm = 0;
     int fwdB = 0;  // batch of the last forward pass (0: none)
     std::vector<void*> allocs;
     std::string msg;
@@ -746,27 +980,32 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
     return FI_OK;
 }
 
+// weight and bias gradients of a pointwise layer: dz x act (NR channels, the last one ones)
+template <int NR>
+int wgrad(fi_fno* h, int B, const bf16* act, long long act_s, int ranges, const int* map, long long base) {
+    const int nz = B * h->ns;
+    k_wgrad<NR><<<std::min(nz, 3 * h->nsm), 256, wgrad_smem<NR>(), h->st>>>(h->dz, act, act_s, h->S2, nz, h->part, h->err,
+                                                                          tc_wait_polls());
+    FNO_CK(cudaGetLastError());
+    FNO_CK(reduce_map(h->part, h->st, nz, C * NR, ranges, map, h->grads, base));
+    return FI_OK;
+}
+
 // gradients of all parameters from dq (and its BF16 copy) set by k_loss
 int backward(fi_fno* h, int B) {
-    const int S = h->S, S2 = h->S2, SL = h->SL, ns = h->ns;
+    const int S = h->S, S2 = h->S2;
     const Offsets& o = h->o;
     const long long vs = (long long)VC * S2, cs = (long long)C * S2;
     float* gr = h->grads;
-    bf16* v4 = h->vext[NLAYER];
-    // projection: recompute the hidden layer, da and GELU(a); weights by split-K over pixels
-    FNO_CK(gemm(h, S2, PW, C, opMN(v4, S2, vs), opK(h->Q1b, C), B,
-                EpiProjBwd{h->params + o.b1, h->params + o.Q2, h->dq, h->da_rows, h->daT, S2}));
-    FNO_CK(gemm(h, 2 * PW, VC, SL, opK(h->daT, S2, (long long)2 * PW * S2, SL), opK(v4, S2, vs, SL), B * ns,
-                EpiStoreF32{h->part, VC, (long long)2 * PW * VC}, ns));
-    FNO_CK(reduce_map(h->part, h->st, B * ns, 2 * PW * VC, 16, h->map_proj, gr, 0));
-    FNO_CK(gemm(h, B * S2, C, PW, opK(h->da_rows, PW), opK(h->Q1Tb, PW), 1, EpiNchw{h->dvf, S2, 0}));
+    const ProjBwdArgs pb{h->vext[NLAYER], h->Q1b, h->Q1Tb, h->params + o.b1, h->params + o.Q2, h->dq, h->dz, h->part, S2,
+                         B * h->ns, h->err, tc_wait_polls()};
+    k_proj_bwd<<<std::min(pb.nslices, 2 * h->nsm), 256, PB_SMEM, h->st>>>(pb);
+    FNO_CK(cudaGetLastError());
+    FNO_CK(reduce_map(h->part, h->st, B * h->ns, PW * VC, 16, h->map_proj, gr, 0));
     for (int l = NLAYER - 1; l >= 0; l--) {
-        k_act_bwd<<<B * (S2 / 64), 256, 0, h->st>>>(h->dvf, l < NLAYER - 1 ? h->zs[l] : nullptr, h->dz, nullptr, S2);
-        FNO_CK(cudaGetLastError());
         // pointwise path weights and bias: [co][ci | ones]
-        FNO_CK(gemm(h, C, C + 1, SL, opK(h->dz, S2, cs, SL), opK(h->vext[l], S2, vs, SL), B * ns,
-                    EpiStoreF32{h->part, C + 1, (long long)C * (C + 1)}, ns));
-        FNO_CK(reduce_map(h->part, h->st, B * ns, C * (C + 1), 32, h->map_loc, gr, o.layer[l]));
+        const int rc = wgrad<C + 1>(h, B, h->vext[l], vs, 32, h->map_loc, o.layer[l]);
+        if (rc) return rc;
         // spectral path: adjoint of the inverse DFT along x, then along y
         FNO_CK(gemm(h, B * C * S, 2 * KX, S, opK(h->dz, S), opK(h->G1T, S), 1, EpiDftX{h->Tb, B, S, 0}));
         FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(h->G2T, 2 * S), 1, EpiModes{h->dYm, B}));
@@ -776,18 +1015,14 @@ int backward(fi_fno* h, int B) {
         FNO_CK(gemm(h, B, 64, 64, opK(h->dYm, 64, (long long)B * 64), opK(h->WmT + (size_t)l * NM * 4096, 64, 4096),
                     NM, EpiMix{h->Yb}));
         FNO_CK(gemm(h, B * C * KX, 2 * S, 64, opK(h->Yb, 64), opK(h->F2T, 64), 1, EpiIdftY{h->Gt, S}));
-        // adjoint of the DFT along x + the pointwise path: batch (b, y), rows x, K = (kx, part) | co
+        // adjoint of the DFT along x + the pointwise path: batch (b, y), rows x, K = (kx, part) | co;
+        // then the activation of the layer below (the lift has none)
         FNO_CK(gemm(h, S, C, 64, opK(h->F1T, 2 * KX), opK(h->Gt, 2 * KX, (long long)S * C * 32, (long long)C * 32),
-                    B * S, EpiPixStore{h->dvf, S, S2}, S, opMN(h->dz, S2, cs, S), opK(h->WlT + (size_t)l * C * C, C),
-                    2 * KX));
+                    B * S, EpiPixBwd{l > 0 ? h->zs[l - 1] : nullptr, h->dz, S, S2}, S, opMN(h->dz, S2, cs, S),
+                    opK(h->WlT + (size_t)l * C * C, C), 2 * KX));
     }
-    // lift weights and bias: [c][inputs | ones | zero]
-    k_act_bwd<<<B * (S2 / 64), 256, 0, h->st>>>(h->dvf, nullptr, h->dz, nullptr, S2);
-    FNO_CK(cudaGetLastError());
-    FNO_CK(gemm(h, C, XC, SL, opK(h->dz, S2, cs, SL), opK(h->xe, S2, (long long)XC * S2, SL), B * ns,
-                EpiStoreF32{h->part, XC, (long long)C * XC}, ns));
-    FNO_CK(reduce_map(h->part, h->st, B * ns, C * XC, 64, h->map_lift, gr, 0));
-    return FI_OK;
+    // lift weights and bias: [c][inputs | ones]
+    return wgrad<NIN + 1>(h, B, h->xe, (long long)XC * S2, 64, h->map_lift, 0);
 }
 
 int set_loss(fi_fno* h, int B, const float* target, const float* w, const float* dy) {
@@ -831,14 +1066,20 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     h->maxB = max_batch;
     h->device = device;
     h->o = offsets();
-    h->SL = 512;  // pixels per split-K slice of the weight gradients (S2 is a multiple of 1024)
-    h->ns = h->S2 / h->SL;
+    h->ns = h->S2 / SLICE;
     auto bad = [&](int rc) {
         fi_fno_destroy(h);
         return rc;
     };
     if (cudaSetDevice(device) != cudaSuccess) return bad(FI_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamDefault) != cudaSuccess) return bad(FI_ERR_CUDA);
+    if (cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaFuncSetAttribute(k_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_wgrad<C + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<C + 1>()) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_wgrad<NIN + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<NIN + 1>()) !=
+            cudaSuccess)
+        return bad(FI_ERR_CUDA);
     const long long B = max_batch, S2 = h->S2, P = h->o.total;
     bool ok = dalloc(h, &h->params, P) == cudaSuccess && dalloc(h, &h->grads, P) == cudaSuccess &&
               dalloc(h, &h->m, P) == cudaSuccess && dalloc(h, &h->v, P) == cudaSuccess &&
@@ -856,13 +1097,11 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
               dalloc(h, &h->Gt, (size_t)B * C * S * 32) == cudaSuccess &&
               dalloc(h, &h->dz, (size_t)B * C * S2) == cudaSuccess &&
               dalloc(h, &h->dYm, (size_t)NM * B * 64) == cudaSuccess &&
-              dalloc(h, &h->da_rows, (size_t)B * S2 * PW) == cudaSuccess &&
-              dalloc(h, &h->daT, (size_t)B * 2 * PW * S2) == cudaSuccess &&
               dalloc(h, &h->q, (size_t)B * S2) == cudaSuccess &&
-              dalloc(h, &h->dq, (size_t)B * S2) == cudaSuccess && dalloc(h, &h->dvf, (size_t)B * C * S2) == cudaSuccess &&
-              dalloc(h, &h->part, (size_t)B * h->ns * 2 * PW * VC) == cudaSuccess &&
+              dalloc(h, &h->dq, (size_t)B * S2) == cudaSuccess &&
+              dalloc(h, &h->part, (size_t)B * h->ns * PW * VC) == cudaSuccess &&
               dalloc(h, &h->scal, 4) == cudaSuccess && dalloc(h, &h->map_loc, C * (C + 1)) == cudaSuccess &&
-              dalloc(h, &h->map_proj, 2 * PW * VC) == cudaSuccess && dalloc(h, &h->map_lift, C * XC) == cudaSuccess &&
+              dalloc(h, &h->map_proj, PW * VC) == cudaSuccess && dalloc(h, &h->map_lift, C * (NIN + 1)) == cudaSuccess &&
               dalloc(h, &h->err, 1) == cudaSuccess;
     for (int l = 0; l <= NLAYER && ok; l++) ok = dalloc(h, &h->vext[l], (size_t)B * VC * S2) == cudaSuccess;
     for (int l = 0; l < NLAYER && ok; l++)
@@ -878,17 +1117,17 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
             return bad(FI_ERR_CUDA);
     // split-K gradient maps (targets relative to the base passed to k_reduce_map)
     const Offsets& o = h->o;
-    std::vector<int> ml(C * (C + 1)), mp(2 * PW * VC, -1), mf(C * XC, -1);
+    std::vector<int> ml(C * (C + 1)), mp(PW * VC), mf(C * (NIN + 1));
     for (int co = 0; co < C; co++)
         for (int k = 0; k <= C; k++) ml[co * (C + 1) + k] = (int)(k < C ? SPEC + co * C + k : SPEC + C * C + co);
     for (int j = 0; j < PW; j++) {
         for (int c = 0; c < C; c++) mp[j * VC + c] = (int)(o.Q1 + j * C + c);
         mp[j * VC + C] = (int)(o.b1 + j);
-        mp[(PW + j) * VC + C + 1] = (int)(o.Q2 + j);
+        mp[j * VC + C + 1] = (int)(o.Q2 + j);
     }
     for (int c = 0; c < C; c++) {
-        for (int k = 0; k < NIN; k++) mf[c * XC + k] = (int)(o.P + c * NIN + k);
-        mf[c * XC + NIN] = (int)(o.bP + c);
+        for (int k = 0; k < NIN; k++) mf[c * (NIN + 1) + k] = (int)(o.P + c * NIN + k);
+        mf[c * (NIN + 1) + NIN] = (int)(o.bP + c);
     }
     if (cudaMemcpy(h->map_loc, ml.data(), ml.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(h->map_proj, mp.data(), mp.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||

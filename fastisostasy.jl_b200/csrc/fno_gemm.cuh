@@ -183,15 +183,18 @@ __device__ __forceinline__ void tc_stage(uint32_t dst, const TcOperand& o1, cons
                                          int row0, int nrows, int k0, int kc, int K, int K1, const void* safe) {
     const int left = nrows - row0;
     // K-major groups: one 16-byte copy = 8 consecutive K elements of one row; a thread keeps its
-    // K group, so its operand and column are fixed
+    // K group, so its operand and column are fixed.  Eight neighbouring threads take the eight rows
+    // of one core matrix (contiguous in shared memory: no bank conflicts), the next eight the next
+    // K group (contiguous in global memory).
     if (!(o1.mn && o2.mn)) {
         const int sh = kc <= 16 ? 1 : kc <= 32 ? 2 : 3;
-        const int kv = threadIdx.x & ((1 << sh) - 1), gk = k0 + kv * 8;
+        const int kv = (threadIdx.x >> 3) & ((1 << sh) - 1), gk = k0 + kv * 8;
         const bool second = gk >= K1;
         const TcOperand& o = second ? o2 : o1;
         if (!o.mn && (second ? do2 : do1) && kv * 8 < kc) {
             const bool kok = gk < K;
-            const int r_ = threadIdx.x >> sh, step = NTHR >> sh, rows = left < ROWS ? left : ROWS;
+            const int r_ = (threadIdx.x >> (3 + sh)) * 8 + (threadIdx.x & 7), step = NTHR >> sh;
+            const int rows = left < ROWS ? left : ROWS;
             const __nv_bfloat16* src = o.p + (size_t)z1 * o.s + (size_t)z2 * o.s2 + (second ? gk - K1 : gk) +
                                        (size_t)(row0 + r_) * o.ld;
             const size_t sstep = (size_t)step * o.ld;
@@ -200,11 +203,12 @@ __device__ __forceinline__ void tc_stage(uint32_t dst, const TcOperand& o1, cons
         }
     }
     // MN-major groups: one 16-byte copy = 8 consecutive rows of one K column, stored as
-    // row (k % 8) of core matrix (k / 8, r / 8)
+    // row (k % 8) of core matrix (k / 8, r / 8); eight neighbouring threads take the eight columns of
+    // one core matrix
     if (o1.mn || o2.mn) {
         constexpr int RV = ROWS / 8;
         for (int v = threadIdx.x; v < RV * kc; v += NTHR) {
-            const int kc_ = v / RV, rv = v - kc_ * RV;
+            const int rv = (v >> 3) % RV, kc_ = v / (8 * RV) * 8 + (v & 7);
             const int gk = k0 + kc_;
             const bool second = gk >= K1;
             const TcOperand& o = second ? o2 : o1;
