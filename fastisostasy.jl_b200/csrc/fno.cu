@@ -285,7 +285,6 @@ __global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ dz, cons
         cp_async_commit();
     };
     int z = blockIdx.x;
-    if (z < nslices) stage(z);
     if (warp == 0) {
         tc_alloc(&tmem_base, 64);
         tc_relinquish();
@@ -298,6 +297,9 @@ __global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ dz, cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    dep_wait();
+    if (dep_early()) dep_launch();
+    if (z < nslices) stage(z);
     const uint32_t tmem = tmem_base;
     int n = 0;  // slices committed
     for (; z < nslices; z += gridDim.x) {
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ dz, cons
         }
         // the next slice's MMAs are issued after the next __syncthreads()
     }
+    if (!dep_early()) dep_launch();
     cp_async_wait<0>();
     if (s_fail && tid == 0) {
         if (err) atomicExch(err, FI_ERR_TIMEOUT);
@@ -399,19 +402,6 @@ __global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ Pro
     };
     const int my = g.nslices > (int)blockIdx.x ? (g.nslices - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const int ntiles = 4 * my;
-    for (int v = tid; v < PW * 4; v += 256) {
-        const int r = v >> 2, q = v & 3;
-        cp_async16(s0 + PB_Q1 + q * (PW * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1 + r * C + 8 * q, true);
-    }
-    for (int v = tid; v < C * 16; v += 256) {
-        const int r = v >> 4, q = v & 15;
-        cp_async16(s0 + PB_Q1T + q * (C * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1T + r * PW + 8 * q, true);
-    }
-    if (tid < PW) {
-        sb1[tid] = g.b1[tid];
-        sQ2[tid] = g.Q2[tid];
-    }
-    if (ntiles > 0) stage(0);
     if (warp == 0) {
         tc_alloc(&tmem_base, 256);
         tc_relinquish();
@@ -425,6 +415,21 @@ __global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ Pro
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    dep_wait();
+    if (dep_early()) dep_launch();
+    for (int v = tid; v < PW * 4; v += 256) {
+        const int r = v >> 2, q = v & 3;
+        cp_async16(s0 + PB_Q1 + q * (PW * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1 + r * C + 8 * q, true);
+    }
+    for (int v = tid; v < C * 16; v += 256) {
+        const int r = v >> 4, q = v & 15;
+        cp_async16(s0 + PB_Q1T + q * (C * 16) + (r >> 3) * 128 + (r & 7) * 16, g.Q1T + r * PW + 8 * q, true);
+    }
+    if (tid < PW) {
+        sb1[tid] = g.b1[tid];
+        sQ2[tid] = g.Q2[tid];
+    }
+    if (ntiles > 0) stage(0);
     const uint32_t tmem = tmem_base, tW1 = tmem + PW, tW2 = tmem + PW + 48;
     const int quad = warp & 3, half = warp >> 2, pr = quad * 32 + lane;  // pixel row of the tile, column half
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
@@ -533,6 +538,7 @@ __global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ Pro
         tc_fence_before();
         // the next tile's MMAs are issued after the next __syncthreads()
     }
+    if (!dep_early()) dep_launch();
     cp_async_wait<0>();
     if (s_fail && tid == 0) {
         if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
@@ -549,6 +555,8 @@ __global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ Pro
 
 // x [B][6][S2] FP32 -> NCHW [b][8][S2] BF16 (channel 6 = 1 for the lift's bias gradient)
 __global__ void k_prep_input(const float* __restrict__ x, bf16* xe, int B, int S2) {
+    dep_wait();
+    dep_launch();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)B * S2) return;
     const int b = (int)(i / S2), p = (int)(i - (size_t)b * S2);
@@ -574,6 +582,8 @@ __global__ void k_fill_channel(bf16* v, int B, int S2, int ch, float value) {
 __global__ void __launch_bounds__(256) k_loss(const float* __restrict__ q, const float* __restrict__ target,
                                               const float* __restrict__ w, const float* __restrict__ dy, int n,
                                               int S2, float inv_n, float* dq, bf16* vext4, float* part) {
+    dep_wait();
+    dep_launch();
     const int i = blockIdx.x * 256 + threadIdx.x;
     float l = 0.f, d = 0.f;
     if (i < n) {
@@ -612,6 +622,8 @@ __global__ void __launch_bounds__(256) k_loss(const float* __restrict__ q, const
 // the per-block partials of k_loss summed in a fixed order (one block): the loss and the
 // output-bias gradient come out the same on every run
 __global__ void __launch_bounds__(256) k_loss_sum(const float* __restrict__ part, int nblk, float* loss, float* gb2) {
+    dep_wait();
+    dep_launch();
     __shared__ float sl[256], sd[256];
     float a = 0.f, c = 0.f;
     for (int i = threadIdx.x; i < nblk; i += 256) {
@@ -629,7 +641,7 @@ __global__ void __launch_bounds__(256) k_loss_sum(const float* __restrict__ part
     }
     if (threadIdx.x == 0) {
         *loss = sl[0];
-        *gb2 += sd[0];
+        *gb2 = sd[0];
     }
 }
 
@@ -638,6 +650,8 @@ __global__ void __launch_bounds__(256) k_loss_sum(const float* __restrict__ part
 //   dWi[ci][co] = sum_b dYi[co] Zr[ci] - dYr[co] Zi[ci]
 __global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* __restrict__ Z, const bf16* __restrict__ dY,
                                                     float* gW, int B) {
+    dep_wait();
+    dep_launch();
     __shared__ float zs[64][64], ds[64][64];
     const int mode = blockIdx.x, tid = threadIdx.x;
     float sr[4] = {0.f, 0.f, 0.f, 0.f}, si[4] = {0.f, 0.f, 0.f, 0.f};
@@ -668,12 +682,14 @@ __global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* __restrict__ Z, 
     }
 }
 
-// split-K partials [z][MN] summed over z and added to grad[base + map[i]] (grad is zeroed before the
-// backward pass; map is one-to-one), in a fixed order, so that gradients are the same on every run:
+// split-K partials [z][MN] summed over z into grad[base + map[i]] (map is one-to-one; a backward pass
+// writes every gradient once), in a fixed order, so that gradients are the same on every run:
 // each of at most 64 ranges of `per` consecutive z in order (range y and y + 32 by row y of the
 // block), then the ranges in order.
 __global__ void __launch_bounds__(1024) k_reduce_map(const float* __restrict__ part, int nz, int MN, int per,
                                                      const int* __restrict__ map, float* grad, long long base) {
+    dep_wait();
+    dep_launch();
     __shared__ float sm[64][33];
     const int i = blockIdx.x * 32 + threadIdx.x;
     for (int y = threadIdx.y; y < 64; y += 32) {
@@ -689,19 +705,21 @@ __global__ void __launch_bounds__(1024) k_reduce_map(const float* __restrict__ p
     if (threadIdx.y == 0 && i < MN) {
         float a = 0.f;
         for (int y = 0; y * per < nz; y++) a += sm[y][threadIdx.x];
-        grad[base + map[i]] += a;
+        grad[base + map[i]] = a;
     }
 }
 
 // ranges: at most this many (<= 64)
 static cudaError_t reduce_map(const float* part, cudaStream_t st, int nz, int MN, int ranges, const int* map,
                               float* grad, long long base) {
-    k_reduce_map<<<(MN + 31) / 32, dim3(32, 32), 0, st>>>(part, nz, MN, (nz + ranges - 1) / ranges, map, grad, base);
-    return cudaGetLastError();
+    return launch_dep(k_reduce_map, (MN + 31) / 32, dim3(32, 32), 0, st, part, nz, MN, (nz + ranges - 1) / ranges, map, grad,
+                      base);
 }
 
 __global__ void k_adam(float* p, const float* __restrict__ g, float* m, float* v, long long n, float lr, float b1,
                        float b2, float eps, float c1, float c2) {
+    dep_wait();
+    dep_launch();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -717,6 +735,8 @@ __global__ void k_adam(float* p, const float* __restrict__ g, float* m, float* v
 // both matrices written along their rows, through a shared-memory copy of the mode.
 __global__ void __launch_bounds__(256) k_pack_spec(const float* __restrict__ params, long long off0, bf16* Wm,
                                                    bf16* WmT) {
+    dep_wait();
+    dep_launch();
     __shared__ float w[2][C][C + 1];  // [re, im][ci][co]
     const int mode = blockIdx.x, l = blockIdx.y;
     const float* W = params + off0 + (long long)l * LAYER + (size_t)mode * 2 * C * C;
@@ -738,6 +758,8 @@ __global__ void __launch_bounds__(256) k_pack_spec(const float* __restrict__ par
 // pointwise weights -> BF16 operands: P [32][8], Wloc [l][co][ci] and [l][ci][co], Q1 [128][32], [32][128]
 __global__ void k_pack_small(const float* __restrict__ params, Offsets o, bf16* Pb, bf16* Wl, bf16* WlT, bf16* Q1b,
                              bf16* Q1Tb) {
+    dep_wait();
+    dep_launch();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < C * XC) {
         const int c = i / XC, k = i - c * XC;
@@ -933,17 +955,18 @@ void build_dft(int S, std::vector<bf16> (&mats)[8]) {
 }
 
 int pack(fi_fno* h) {
-    k_pack_spec<<<dim3(NM, NLAYER), 256, 0, h->st>>>(h->params, h->o.layer[0], h->Wm, h->WmT);
-    k_pack_small<<<(PW * C + 255) / 256, 256, 0, h->st>>>(h->params, h->o, h->Pb, h->Wl, h->WlT, h->Q1b, h->Q1Tb);
-    FNO_CK(cudaGetLastError());
+    FNO_CK(launch_dep(k_pack_spec, dim3(NM, NLAYER), 256, 0, h->st, h->params, h->o.layer[0], h->Wm, h->WmT));
+    FNO_CK(launch_dep(k_pack_small, (PW * C + 255) / 256, 256, 0, h->st, h->params, h->o, h->Pb, h->Wl, h->WlT, h->Q1b,
+                      h->Q1Tb));
     return FI_OK;
 }
 
-// wait for the stream and read the GEMMs' timeout flag
-int finish(fi_fno* h) {
-    FNO_CK(cudaStreamSynchronize(h->st));
+// wait for the stream; read the GEMMs' timeout flag and, if asked, the loss
+int finish(fi_fno* h, float* loss = nullptr) {
     int e = 0;
-    FNO_CK(cudaMemcpy(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost));
+    FNO_CK(cudaMemcpyAsync(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+    if (loss) FNO_CK(cudaMemcpyAsync(loss, h->scal, sizeof(float), cudaMemcpyDeviceToHost, h->st));
+    FNO_CK(cudaStreamSynchronize(h->st));
     if (e) return fail(h, e, "a tensor-core GEMM wait gave up");
     return FI_OK;
 }
@@ -984,9 +1007,8 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
 template <int NR>
 int wgrad(fi_fno* h, int B, const bf16* act, long long act_s, int ranges, const int* map, long long base) {
     const int nz = B * h->ns;
-    k_wgrad<NR><<<std::min(nz, 3 * h->nsm), 256, wgrad_smem<NR>(), h->st>>>(h->dz, act, act_s, h->S2, nz, h->part, h->err,
-                                                                          tc_wait_polls());
-    FNO_CK(cudaGetLastError());
+    FNO_CK(launch_dep(k_wgrad<NR>, std::min(nz, 3 * h->nsm), 256, wgrad_smem<NR>(), h->st, h->dz, act, act_s, h->S2, nz,
+                      h->part, h->err, tc_wait_polls()));
     FNO_CK(reduce_map(h->part, h->st, nz, C * NR, ranges, map, h->grads, base));
     return FI_OK;
 }
@@ -999,8 +1021,7 @@ int backward(fi_fno* h, int B) {
     float* gr = h->grads;
     const ProjBwdArgs pb{h->vext[NLAYER], h->Q1b, h->Q1Tb, h->params + o.b1, h->params + o.Q2, h->dq, h->dz, h->part, S2,
                          B * h->ns, h->err, tc_wait_polls()};
-    k_proj_bwd<<<std::min(pb.nslices, 2 * h->nsm), 256, PB_SMEM, h->st>>>(pb);
-    FNO_CK(cudaGetLastError());
+    FNO_CK(launch_dep(k_proj_bwd, std::min(pb.nslices, 2 * h->nsm), 256, PB_SMEM, h->st, pb));
     FNO_CK(reduce_map(h->part, h->st, B * h->ns, PW * VC, 16, h->map_proj, gr, 0));
     for (int l = NLAYER - 1; l >= 0; l--) {
         // pointwise path weights and bias: [co][ci | ones]
@@ -1009,8 +1030,7 @@ int backward(fi_fno* h, int B) {
         // spectral path: adjoint of the inverse DFT along x, then along y
         FNO_CK(gemm(h, B * C * S, 2 * KX, S, opK(h->dz, S), opK(h->G1T, S), 1, EpiDftX{h->Tb, B, S, 0}));
         FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(h->G2T, 2 * S), 1, EpiModes{h->dYm, B}));
-        k_spec_wgrad<<<NM, 256, 0, h->st>>>(h->Zm[l], h->dYm, gr + o.layer[l], B);
-        FNO_CK(cudaGetLastError());
+        FNO_CK(launch_dep(k_spec_wgrad, NM, 256, 0, h->st, h->Zm[l], h->dYm, gr + o.layer[l], B));
         // adjoint of the channel mixing and of the DFT along y
         FNO_CK(gemm(h, B, 64, 64, opK(h->dYm, 64, (long long)B * 64), opK(h->WmT + (size_t)l * NM * 4096, 64, 4096),
                     NM, EpiMix{h->Yb}));
@@ -1027,13 +1047,11 @@ int backward(fi_fno* h, int B) {
 
 int set_loss(fi_fno* h, int B, const float* target, const float* w, const float* dy) {
     const int n = B * h->S2;
-    FNO_CK(cudaMemsetAsync(h->grads, 0, sizeof(float) * h->o.total, h->st));
-    FNO_CK(cudaMemsetAsync(h->scal, 0, sizeof(float) * 4, h->st));
     // per-block partials in the split-K scratch (free until the backward pass)
     const int nblk = (n + 255) / 256;
-    k_loss<<<nblk, 256, 0, h->st>>>(h->q, target, w, dy, n, h->S2, 1.f / n, h->dq, h->vext[NLAYER], h->part);
-    k_loss_sum<<<1, 256, 0, h->st>>>(h->part, nblk, h->scal, h->grads + h->o.b2);
-    FNO_CK(cudaGetLastError());
+    FNO_CK(launch_dep(k_loss, nblk, 256, 0, h->st, h->q, target, w, dy, n, h->S2, 1.f / n, h->dq, h->vext[NLAYER],
+                      h->part));
+    FNO_CK(launch_dep(k_loss_sum, 1, 256, 0, h->st, h->part, nblk, h->scal, h->grads + h->o.b2));
     return FI_OK;
 }
 
@@ -1041,9 +1059,8 @@ int adam(fi_fno* h, float lr) {
     h->adam_t++;
     const float c1 = (float)(1.0 / (1.0 - std::pow((double)h->beta1, (double)h->adam_t)));
     const float c2 = (float)(1.0 / (1.0 - std::pow((double)h->beta2, (double)h->adam_t)));
-    k_adam<<<148 * 8, 256, 0, h->st>>>(h->params, h->grads, h->m, h->v, h->o.total, lr, h->beta1, h->beta2, h->eps,
-                                       c1, c2);
-    FNO_CK(cudaGetLastError());
+    FNO_CK(launch_dep(k_adam, 148 * 8, 256, 0, h->st, h->params, h->grads, h->m, h->v, h->o.total, lr, h->beta1, h->beta2,
+                      h->eps, c1, c2));
     return pack(h);
 }
 
@@ -1207,8 +1224,7 @@ int fi_fno_train_step_weighted(fi_fno* h, int32_t B, const float* x, const float
     if (!rc) rc = set_loss(h, B, target, w, nullptr);
     if (!rc) rc = backward(h, B);
     if (!rc) rc = adam(h, lr);
-    if (!rc) rc = finish(h);
-    if (!rc && loss) FNO_CK(cudaMemcpy(loss, h->scal, sizeof(float), cudaMemcpyDeviceToHost));
+    if (!rc) rc = finish(h, loss);
     return rc;
 }
 
@@ -1220,8 +1236,7 @@ int fi_fno_loss_backward(fi_fno* h, int32_t B, const float* x, const float* targ
     rc = forward(h, B, x, h->q);
     if (!rc) rc = set_loss(h, B, target, w, nullptr);
     if (!rc) rc = backward(h, B);
-    if (!rc) rc = finish(h);
-    if (!rc && loss) FNO_CK(cudaMemcpy(loss, h->scal, sizeof(float), cudaMemcpyDeviceToHost));
+    if (!rc) rc = finish(h, loss);
     return rc;
 }
 

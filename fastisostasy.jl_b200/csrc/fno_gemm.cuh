@@ -128,6 +128,38 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch: a kernel's blocks may start while the kernel before it in the
+// stream still runs.  Each one calls dep_wait() before its first access to global memory that
+// another kernel touches (it returns when the kernels before have completed and their writes are
+// visible).  It calls dep_launch() after that -- and after it has its tensor memory, which a waiting
+// block of the next kernel must not hold in its place: at once if the grid has at most one block
+// an SM (dep_early), else when its tiles are done.  (Blocks of the next kernel that start early
+// gather on the SMs that are free first and then walk their equal shares there: 32 samples of
+// 128 x 128, inference 659 us with the late call, 793 with the early one, 695 without.)  What
+// overlaps is the launch latency and the prologue.  One 64 x 64 sample: 228 -> 170 us; training
+// step of 7 samples of 96 x 96: 768 -> 612 us.
+// ---------------------------------------------------------------------------
+constexpr unsigned DEP_EARLY_BLOCKS = 148;
+__device__ __forceinline__ bool dep_early() { return gridDim.x <= DEP_EARLY_BLOCKS; }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------
 // One GEMM operand.  K-major (mn = 0): element (r, k) of batch (z1, z2) at
@@ -267,7 +299,6 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
         cp_async_commit();
     };
     unsigned tile = blockIdx.x;
-    if (tile < ntiles) stage(tile, 0, 0, true);
     if (warp == 0) {
         tc_alloc(&tmem_base, BN < 32 ? 32 : BN);
         tc_relinquish();
@@ -281,6 +312,9 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    dep_wait();
+    if (dep_early()) dep_launch();
+    if (tile < ntiles) stage(tile, 0, 0, true);
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = tc_instr_desc(TC_BM, BN);
     int j = 0;  // chunks so far over all tiles; chunk j uses buffer j % NB
@@ -340,6 +374,7 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
         tc_fence_before();
         __syncthreads();  // the next tile's MMAs overwrite the accumulator
     }
+    if (!dep_early()) dep_launch();
     cp_async_wait<0>();
     if (s_fail && tid == 0) {
         if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
@@ -418,8 +453,8 @@ inline cudaError_t launch_gemm_nb(const TcGemmArgs& g, int batch, const Epi& epi
         (long long)((g.M + TC_BM - 1) / TC_BM) * ((g.N + BN - 1) / BN) * (long long)batch;
     if (ntiles <= 0) return cudaSuccess;
     if (ntiles * ((g.K + TC_BK - 1) / TC_BK) > 0x3fffffffLL) return cudaErrorInvalidValue;
-    k_gemm_tc<BN, NTHR, NB, Epi><<<(unsigned)std::min<long long>(ntiles, blocks), NTHR, smem, st>>>(a, epi);
-    return cudaGetLastError();
+    return launch_dep(k_gemm_tc<BN, NTHR, NB, Epi>, dim3((unsigned)std::min<long long>(ntiles, blocks)), dim3(NTHR), smem,
+                      st, a, epi);
 }
 template <int BN, int NTHR, class Epi>
 inline cudaError_t launch_gemm_tc(const TcGemmArgs& g, int batch, const Epi& epi, cudaStream_t st) {
