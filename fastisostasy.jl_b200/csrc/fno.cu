@@ -14,7 +14,7 @@
 //   DFT along x:   v[(b,c,y)][x]            x F1[(part,kx)][x]            -> T
 //   DFT along y:   T[(kx,b,c)][(part,y)]    x F2[(kyi,part')][(part,y)]   -> Z (per mode)
 //   channel mix:   Z[mode][b][(part,ci)]    x Wmat[mode][(part',co)][(part,ci)]  (512 batches)
-//   inverse y:     Y[(b,co,kx)][(kyi,part)] x G2[(part',y)][(kyi,part)]   -> G[(b,y)][co][(kx,part)]
+//   inverse y:     Y[(b,co,kx)][(kyi,part)] x G2[(y,part')][(kyi,part)]   -> G[(b,y)][co][(kx,part)]
 //   inverse x + pointwise path, one GEMM per row (b, y) of pixels x channels with K = 32 + 32:
 //                  [G1[x][(kx,part)] | v[b][ci][y][x]]  x  [G[(b,y)][co][(kx,part)] | Wloc[co][ci]]
 //                  (the activation v read in place from NCHW as an MN-major operand)
@@ -105,6 +105,7 @@ __device__ __forceinline__ void store16(bf16* dst, const float* v) {
 
 // lift: batch z = b, row p, col c -> v0 in NCHW
 struct EpiLift {
+    static constexpr bool PAIR = false;
     bf16* vext;
     const float* bias;
     int S2;
@@ -116,24 +117,14 @@ struct EpiLift {
     __device__ __forceinline__ void row_done(int, int) const {}
 };
 
-// DFT along x and the adjoint of the inverse along x: col n = part*16 + kx,
-// out T[kx][b][c][part][y].  per_sample: batch z = b and row = (c, y); else row = (b, c, y).
+// DFT along x and the adjoint of the inverse along x: batch z = b, row (c, y), col n = part*16 + kx,
+// out T[kx][b][c][part][y]
 struct EpiDftX {
+    static constexpr bool PAIR = false;
     bf16* T;
-    int B, S, per_sample;
-    __device__ __forceinline__ void operator()(int z, int row, int n0, const float* v, int) const {
-        int b, c, y;
-        if (per_sample) {
-            b = z;
-            c = row / S;
-            y = row - c * S;
-        } else {
-            const int bc = row / S;
-            y = row - bc * S;
-            b = bc / C;
-            c = bc - b * C;
-        }
-        const int part = n0 >> 4;
+    int B, S;
+    __device__ __forceinline__ void operator()(int b, int row, int n0, const float* v, int) const {
+        const int c = row / S, y = row - c * S, part = n0 >> 4;
 #pragma unroll
         for (int i = 0; i < 16; i++)
             T[(((size_t)i * B + b) * C + c) * 2 * S + part * S + y] = __float2bfloat16_rn(v[i]);
@@ -144,6 +135,7 @@ struct EpiDftX {
 // DFT along y (and the adjoint of the inverse along y): row (kx, b, c), col n = kyi*2 + part,
 // out Z[kx*KY + kyi][b][part*32 + c]
 struct EpiModes {
+    static constexpr bool PAIR = false;
     bf16* Z;
     int B;
     __device__ __forceinline__ void operator()(int, int row, int n0, const float* v, int) const {
@@ -157,32 +149,31 @@ struct EpiModes {
     __device__ __forceinline__ void row_done(int, int) const {}
 };
 
-// channel mixing (forward and adjoint): batch z = mode, row b, col n = part*32 + c,
+// channel mixing (forward and adjoint): batch z = mode, row b, cols c (real) and 32 + c (imaginary),
 // out Y[b][c][kx][kyi*2 + part]
 struct EpiMix {
+    static constexpr bool PAIR = true;
     bf16* Y;
-    __device__ __forceinline__ void operator()(int z, int row, int n0, const float* v, int) const {
+    __device__ __forceinline__ void pair(int z, int row, int c0, const float* re, const float* im) const {
         const int kx = z / KY, kyi = z - kx * KY;
+        bf16* y = Y + (((size_t)row * C + c0) * KX + kx) * 64 + kyi * 2;
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int n = n0 + i, part = n >> 5, c = n & 31;
-            Y[(((size_t)row * C + c) * KX + kx) * 64 + kyi * 2 + part] = __float2bfloat16_rn(v[i]);
-        }
+        for (int i = 0; i < 16; i++) *(uint32_t*)(y + (size_t)i * KX * 64) = pack2(re[i], im[i]);
     }
     __device__ __forceinline__ void row_done(int, int) const {}
 };
 
-// inverse DFT along y (and the adjoint of the DFT along y): row (b, c, kx), col n = part*S + y,
+// inverse DFT along y (and the adjoint of the DFT along y): row (b, c, kx), col n = y*2 + part,
 // out G[(b, y)][c][kx*2 + part]
 struct EpiIdftY {
+    static constexpr bool PAIR = false;
     bf16* G;
     int S;
     __device__ __forceinline__ void operator()(int, int row, int n0, const float* v, int) const {
         const int bc = row / KX, kx = row - bc * KX, b = bc / C, c = bc - b * C;
-        const int part = n0 / S, y0 = n0 - part * S;
+        bf16* g = G + (((size_t)b * S + (n0 >> 1)) * C + c) * 32 + kx * 2;
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-            G[(((size_t)b * S + y0 + i) * C + c) * 32 + kx * 2 + part] = __float2bfloat16_rn(v[i]);
+        for (int i = 0; i < 8; i++) *(uint32_t*)(g + (size_t)i * C * 32) = pack2(v[2 * i], v[2 * i + 1]);
     }
     __device__ __forceinline__ void row_done(int, int) const {}
 };
@@ -190,6 +181,7 @@ struct EpiIdftY {
 // inverse DFT along x + pointwise path + bias: batch z = (b, y), row x, col c.  Saves z
 // (FP32) and writes the activation, both NCHW.
 struct EpiPixAct {
+    static constexpr bool PAIR = false;
     const float* bias;
     float* zs;
     bf16* vext;
@@ -213,6 +205,7 @@ struct EpiPixAct {
 // (identity when zs is null) -> dz[b][c][y*S + x] in BF16.  dz may be the operand that the product
 // read: a tile's pixels are read by that tile alone, before its epilogue.
 struct EpiPixBwd {
+    static constexpr bool PAIR = false;
     const float* zs;
     bf16* dz;
     int S, S2;
@@ -230,6 +223,7 @@ struct EpiPixBwd {
 
 // projection: batch z = b, row p, col j (all 128 in one tile): q = sum_j GELU(a_j + b1_j) Q2_j + b2
 struct EpiProj {
+    static constexpr bool PAIR = false;
     const float* b1;
     const float* Q2;
     const float* b2;
@@ -242,6 +236,157 @@ struct EpiProj {
     }
     __device__ __forceinline__ void row_done(int z, int p) { q[(size_t)z * S2 + p] = acc + b2[0]; }
 };
+
+// ---------------------------------------------------------------------------
+// DFT along x and then y of CH channels of a sample (and the adjoint of the inverse), fused:
+//   T[(c, y)][(part, kx)] = v[c][y][x] x F1[(part, kx)][x]          in tiles of 128 rows (c, y)
+//   Z[mode][b][part*32 + c] = T[(c, kx)][(part, y)] x F2[(kyi, part')][(part, y)]
+// T exists only as the BF16 operand of the second product in shared memory: a row's 16 values of a
+// part are two 16-byte pieces of eight (c, kx) at column (part, y), the MN-major core matrices.  For
+// S <= 128 (both operands and two tiles of v fit an SM: 168 KB at 128); wider grids run the two
+// products of the general kernel.  CH is 8 (all 128 rows of the second product) where that gives
+// enough blocks, else fewer.  32 samples of 128 x 128: 40 us in two kernels -> 28 us (caches
+// flushed); one 64 x 64 sample: inference 170 -> 140 us.
+// ---------------------------------------------------------------------------
+constexpr int DFT2_S = 128;
+constexpr int DFT2_NB = 3;  // tile buffers: two tiles' copies in flight
+struct Dft2Args {
+    const bf16 *v, *F1, *F2;
+    long long vs;  // sample stride; channels are S*S apart
+    bf16* Z;
+    int B, S, CH;
+    int* err;
+    long long polls;
+};
+inline int dft2_smem(int S) { return DFT2_NB * 256 * S + 64 * S + 512 * S + 256 * S; }
+
+__global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = g.S, CH = g.CH;
+    const int groups = C / CH, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * CH;
+    const int rows = CH * S, nt = (rows + 127) >> 7, kg = S >> 3;
+    const uint32_t sV = tc_smem_u32(smem), sF1 = sV + DFT2_NB * 256 * S, sA = sF1 + 64 * S, sF2 = sA + 512 * S;
+    // 16-byte pieces of a K-major operand of R rows (row pitch ld): eight neighbouring threads take
+    // the rows of one core matrix, the next eight the next eight columns
+    auto stage = [&](uint32_t dst, const bf16* src, int R, int n, int ld, int kgr) {
+        const int total = ((n + 7) >> 3) * 8 * kgr;
+        for (int v = tid; v < total; v += 256) {
+            const int q = v >> 3, rg = q / kgr, k = q - rg * kgr, r = rg * 8 + (v & 7);
+            if (r < n) cp_async16(dst + k * (R * 16) + rg * 128 + (v & 7) * 16, src + (size_t)r * ld + 8 * k, true);
+        }
+    };
+    stage(sF1, g.F1, 32, 32, S, kg);
+    stage(sF2, g.F2, 64, 64, 2 * S, 2 * kg);
+    if (warp == 0) {
+        tc_alloc(&tmem_base, 128);
+        tc_relinquish();
+    }
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_fail = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base, tD2 = tmem + 64;
+    const bf16* src = g.v + (size_t)b * g.vs + (size_t)c0 * S * S;
+    dep_wait();
+    if (dep_early()) dep_launch();
+    // tile t to buffer t % DFT2_NB; a group is committed for every tile, also past the end
+    auto stage_tile = [&](int t) {
+        if (t < nt) stage(sV + (t % DFT2_NB) * 256 * S, src + (size_t)t * 128 * S, 128, min(128, rows - t * 128), S, kg);
+        cp_async_commit();
+    };
+    for (int t = 0; t < DFT2_NB - 1; t++) stage_tile(t);
+    const int quad = warp & 3, half = warp >> 2, pr = quad * 32 + lane;
+    const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+    int n = 0;  // commits
+    for (int t = 0; t < nt; t++) {
+        stage_tile(t + DFT2_NB - 1);  // its buffer was last read by tile t - 1's product, which is done
+        cp_async_wait<DFT2_NB - 1>();
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            const uint32_t a0 = sV + (t % DFT2_NB) * 256 * S;
+            for (int ks = 0; ks < S / 16; ks++)
+                tc_mma(tmem, tc_smem_desc(a0 + 2 * ks * 2048, 2048, 128), tc_smem_desc(sF1 + 2 * ks * 512, 512, 128),
+                       tc_instr_desc(TC_BM, 32), ks > 0);
+            tc_commit(&bar);
+            if (!mbar_wait(&bar, (uint32_t)(n & 1), g.polls)) s_fail = 1;
+        }
+        n++;
+        __syncthreads();
+        if (s_fail) break;
+        tc_fence_after();
+        // this thread's row (c, y), part `half`
+        float v[16];
+        tc_ld16(tmem + lanes + (uint32_t)(half * 16), v);
+        const int row = t * 128 + pr;
+        if (row < rows) {
+            const int c = row / S, k = half * S + row - c * S;
+            unsigned char* d = smem + (sA - sV) + (k >> 3) * 2048 + (2 * c) * 128 + (k & 7) * 16;
+            *(uint4*)d = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+            *(uint4*)(d + 128) = make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
+        }
+        tc_fence_before();
+    }
+    if (!s_fail) {
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            for (int ks = 0; ks < S / 8; ks++)
+                tc_mma(tD2, tc_smem_desc(sA + 2 * ks * 2048, 2048, 128), tc_smem_desc(sF2 + 2 * ks * 1024, 1024, 128),
+                       tc_instr_desc(TC_BM, 64) | (1u << 15), ks > 0);
+            tc_commit(&bar);
+            if (!mbar_wait(&bar, (uint32_t)(n & 1), g.polls)) s_fail = 1;
+        }
+        n++;
+        __syncthreads();
+    }
+    if (!s_fail) {
+        if (!dep_early()) dep_launch();
+        tc_fence_after();
+        // row m = (c, kx): to shared memory as [kx][kyi][part][c] (the tiles of v are done), then out in
+        // runs of CH channels
+        bf16* const zt = (bf16*)smem;
+        const int kxp = 64 * CH + 8;  // pitch of a kx: its rows start in different banks
+        const int c = pr >> 4, kx = pr & 15;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            float v[16];
+            tc_ld16(tD2 + lanes + (uint32_t)(half * 32 + q * 16), v);
+            if (c < CH) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) zt[kx * kxp + (half * 32 + q * 16 + i) * CH + c] = __float2bfloat16_rn(v[i]);
+            }
+        }
+        tc_fence_before();
+        __syncthreads();
+        for (int v = tid; v < KX * 64; v += 256) {
+            const int k = v >> 6, r = v & 63;  // r = kyi*2 + part
+            const bf16* z = zt + k * kxp + r * CH;
+            bf16* o = g.Z + ((size_t)(k * KY + (r >> 1)) * g.B + b) * 64 + (r & 1) * 32 + c0;
+            if (CH == 8) *(uint4*)o = *(const uint4*)z;
+            else if (CH == 4) *(uint2*)o = *(const uint2*)z;
+            else if (CH == 2) *(uint32_t*)o = *(const uint32_t*)z;
+            else *o = *z;
+        }
+    }
+    cp_async_wait<0>();
+    if (s_fail && tid == 0) {
+        if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
+        mbar_wait(&bar, (uint32_t)((n - 1) & 1));  // let the issued MMAs finish before their memory goes
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc_dealloc(tmem, 128);
+}
 
 // ---------------------------------------------------------------------------
 // weight gradients of the pointwise layers: slices of SLICE pixels
@@ -931,15 +1076,14 @@ void build_dft(int S, std::vector<bf16> (&mats)[8]) {
     for (auto& m : mats) m.clear();
     mats[0].resize(32 * S);      // F1  [part*16+kx][x]
     mats[1].resize(64 * 2 * S);  // F2  [kyi*2+part'][part*S+y]
-    mats[2].resize(2 * S * 64);  // G2  [part'*S+y][kyi*2+part]
+    mats[2].resize(2 * S * 64);  // G2  [y*2+part'][kyi*2+part]
     mats[3].resize(S * 32);      // G1  [x][kx*2+part]
     mats[4].resize(S * 32);      // F1T [x][kx*2+part]
-    mats[5].resize(2 * S * 64);  // F2T [part*S+y][kyi*2+part']
+    mats[5].resize(2 * S * 64);  // F2T [y*2+part][kyi*2+part']
     mats[6].resize(64 * 2 * S);  // G2T [kyi*2+part][part'*S+y]
     mats[7].resize(32 * S);      // G1T [part*16+kx][x]
     for (size_t i = 0; i < F1.size(); i++) mats[0][i] = bf(F1[i]);
     for (size_t i = 0; i < F2.size(); i++) mats[1][i] = bf(F2[i]);
-    for (size_t i = 0; i < G2.size(); i++) mats[2][i] = bf(G2[i]);
     for (size_t i = 0; i < G1.size(); i++) mats[3][i] = bf(G1[i]);
     for (int x = 0; x < S; x++)
         for (int kx = 0; kx < KX; kx++)
@@ -949,7 +1093,9 @@ void build_dft(int S, std::vector<bf16> (&mats)[8]) {
             }
     for (int r = 0; r < 2 * S; r++)
         for (int n = 0; n < 64; n++) {
-            mats[5][r * 64 + n] = bf(F2[n * 2 * S + r]);
+            const int q = (r % S) * 2 + r / S;  // row (part, y) -> (y, part)
+            mats[2][q * 64 + n] = bf(G2[r * 64 + n]);
+            mats[5][q * 64 + n] = bf(F2[n * 2 * S + r]);
             mats[6][n * 2 * S + r] = bf(G2[r * 64 + n]);
         }
 }
@@ -971,6 +1117,21 @@ int finish(fi_fno* h, float* loss = nullptr) {
     return FI_OK;
 }
 
+// truncated DFT along x and y (F1, F2), or the adjoint of the inverse (G1T, G2T), of 32 channels
+int dft2(fi_fno* h, int B, const bf16* v, long long vs, const bf16* F1, const bf16* F2, bf16* Z) {
+    const int S = h->S;
+    if (S <= DFT2_S) {
+        int CH = 8;
+        while (CH > 1 && B * (C / CH) < 96) CH /= 2;
+        const Dft2Args a{v, F1, F2, vs, Z, B, S, CH, h->err, tc_wait_polls()};
+        FNO_CK(launch_dep(k_dft2, B * (C / CH), 256, dft2_smem(S), h->st, a));
+        return FI_OK;
+    }
+    FNO_CK(gemm(h, C * S, 2 * KX, S, opK(v, S, vs), opK(F1, S), B, EpiDftX{h->Tb, B, S}));
+    FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(F2, 2 * S), 1, EpiModes{Z, B}));
+    return FI_OK;
+}
+
 int forward(fi_fno* h, int B, const float* x, float* y) {
     const int S = h->S, S2 = h->S2;
     const Offsets& o = h->o;
@@ -982,10 +1143,8 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
                 EpiLift{h->vext[0], h->params + o.bP, S2}));
     for (int l = 0; l < NLAYER; l++) {
         const float* lp = h->params + o.layer[l];
-        // DFT along x: per sample, rows (c, y)
-        FNO_CK(gemm(h, C * S, 2 * KX, S, opK(h->vext[l], S, vs), opK(h->F1, S), B, EpiDftX{h->Tb, B, S, 1}));
-        // DFT along y: rows (kx, b, c)
-        FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(h->F2, 2 * S), 1, EpiModes{h->Zm[l], B}));
+        const int rc = dft2(h, B, h->vext[l], vs, h->F1, h->F2, h->Zm[l]);
+        if (rc) return rc;
         // channel mixing, one batch per mode
         FNO_CK(gemm(h, B, 64, 64, opK(h->Zm[l], 64, (long long)B * 64), opK(h->Wm + (size_t)l * NM * 4096, 64, 4096),
                     NM, EpiMix{h->Yb}));
@@ -1025,11 +1184,11 @@ int backward(fi_fno* h, int B) {
     FNO_CK(reduce_map(h->part, h->st, B * h->ns, PW * VC, 16, h->map_proj, gr, 0));
     for (int l = NLAYER - 1; l >= 0; l--) {
         // pointwise path weights and bias: [co][ci | ones]
-        const int rc = wgrad<C + 1>(h, B, h->vext[l], vs, 32, h->map_loc, o.layer[l]);
+        int rc = wgrad<C + 1>(h, B, h->vext[l], vs, 32, h->map_loc, o.layer[l]);
         if (rc) return rc;
         // spectral path: adjoint of the inverse DFT along x, then along y
-        FNO_CK(gemm(h, B * C * S, 2 * KX, S, opK(h->dz, S), opK(h->G1T, S), 1, EpiDftX{h->Tb, B, S, 0}));
-        FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(h->G2T, 2 * S), 1, EpiModes{h->dYm, B}));
+        rc = dft2(h, B, h->dz, cs, h->G1T, h->G2T, h->dYm);
+        if (rc) return rc;
         FNO_CK(launch_dep(k_spec_wgrad, NM, 256, 0, h->st, h->Zm[l], h->dYm, gr + o.layer[l], B));
         // adjoint of the channel mixing and of the DFT along y
         FNO_CK(gemm(h, B, 64, 64, opK(h->dYm, 64, (long long)B * 64), opK(h->WmT + (size_t)l * NM * 4096, 64, 4096),
@@ -1092,6 +1251,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamDefault) != cudaSuccess) return bad(FI_ERR_CUDA);
     if (cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaFuncSetAttribute(k_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_dft2, cudaFuncAttributeMaxDynamicSharedMemorySize, dft2_smem(DFT2_S)) != cudaSuccess ||
         cudaFuncSetAttribute(k_wgrad<C + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<C + 1>()) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_wgrad<NIN + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<NIN + 1>()) !=
@@ -1109,7 +1269,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
               dalloc(h, &h->F1T, 32 * S) == cudaSuccess && dalloc(h, &h->F2T, 128 * S) == cudaSuccess &&
               dalloc(h, &h->G2T, 128 * S) == cudaSuccess && dalloc(h, &h->G1T, 32 * S) == cudaSuccess &&
               dalloc(h, &h->xe, B * XC * S2) == cudaSuccess &&
-              dalloc(h, &h->Tb, (size_t)KX * B * C * 2 * S) == cudaSuccess &&
+              dalloc(h, &h->Tb, S > DFT2_S ? (size_t)KX * B * C * 2 * S : 1) == cudaSuccess &&
               dalloc(h, &h->Yb, (size_t)B * C * KX * 64) == cudaSuccess &&
               dalloc(h, &h->Gt, (size_t)B * C * S * 32) == cudaSuccess &&
               dalloc(h, &h->dz, (size_t)B * C * S2) == cudaSuccess &&

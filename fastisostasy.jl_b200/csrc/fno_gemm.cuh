@@ -365,10 +365,21 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
         Epi e = epi;  // per tile: the epilogue may carry per-row state across its column chunks
         constexpr int CW = NTHR == 256 ? BN / 2 : BN;  // columns a warp reads
         const int quad = warp & 3, cb = (warp >> 2) * CW, row = tm0 + quad * 32 + lane;
-        for (int c0 = cb; c0 < cb + CW; c0 += 16) {
-            float v[16];
-            tc_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
-            if (row < g.M && tn0 + c0 < g.N) e(tz, row, tn0 + c0, v, g.N - (tn0 + c0));
+        if constexpr (Epi::PAIR) {
+            // columns c and c + BN / 2 together (N == BN)
+            static_assert(NTHR == 128, "one warp reads both halves");
+            for (int c0 = 0; c0 < BN / 2; c0 += 16) {
+                float v[16], w[16];
+                tc_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+                tc_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c0 + BN / 2), w);
+                if (row < g.M) e.pair(tz, row, c0, v, w);
+            }
+        } else {
+            for (int c0 = cb; c0 < cb + CW; c0 += 16) {
+                float v[16];
+                tc_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+                if (row < g.M && tn0 + c0 < g.N) e(tz, row, tn0 + c0, v, g.N - (tn0 + c0));
+            }
         }
         if (warp < 4 && row < g.M) e.row_done(tz, row);
         tc_fence_before();
@@ -389,7 +400,11 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
 }
 
 // plain FP32 store: C[z][row][col], pitch ldc
-struct EpiStoreF32 {
+struct EpiBase {
+    static constexpr bool PAIR = false;  // true: pair(z, row, col, v, w) with the columns col and col + BN / 2
+};
+struct EpiStoreF32 : EpiBase {
+    EpiStoreF32(float* C_, int ldc_, long long sC_) : C(C_), ldc(ldc_), sC(sC_) {}
     float* C;
     int ldc;
     long long sC;
@@ -415,9 +430,9 @@ struct EpiStoreF32 {
 // blocks an SM overlap one's epilogue with another's copies and MMAs.  One block per tile kept an
 // SM at 2.7 blocks of 10 that fit (launches could not keep up): inverse x + pointwise product of
 // 32 samples of 128 x 128, 4096 tiles: 83 -> 58 us, its adjoint 60 -> 38 us, lift 48 -> 27 us.
-// Blocks an SM, us per inference / training step of that batch: 2 857 / 2486, 4 728 / 2200, 6 710 /
-// 2191, 8 717 / 2212, 12 722 / 2228 (one block per tile: 801 / 2449).
-constexpr int TC_BLOCKS_SM = 6;
+// Blocks an SM, us per inference / training step of that batch (final kernels): 4 614 / 1500, 6 619 /
+// 1503, 8 603 / 1485, 10 596 / 1475.
+constexpr int TC_BLOCKS_SM = 10;
 template <int BN, int NTHR, int NB, class Epi>
 inline cudaError_t launch_gemm_nb(const TcGemmArgs& g, int batch, const Epi& epi, cudaStream_t st) {
     const int kc0 = g.K < TC_BK ? (g.K + 15) & ~15 : TC_BK;
@@ -464,9 +479,10 @@ inline cudaError_t launch_gemm_tc(const TcGemmArgs& g, int batch, const Epi& epi
 // Tile width by N; 256 threads where the tile is 128 columns wide.
 template <class Epi>
 inline cudaError_t launch_gemm(const TcGemmArgs& g, int batch, const Epi& epi, cudaStream_t st) {
-    if (g.N <= 32) return launch_gemm_tc<32, 128>(g, batch, epi, st);
-    if (g.N <= 64) return launch_gemm_tc<64, 128>(g, batch, epi, st);
-    return launch_gemm_tc<128, 256>(g, batch, epi, st);
+    if constexpr (Epi::PAIR) return launch_gemm_tc<64, 128>(g, batch, epi, st);  // N == 64
+    else if (g.N <= 32) return launch_gemm_tc<32, 128>(g, batch, epi, st);
+    else if (g.N <= 64) return launch_gemm_tc<64, 128>(g, batch, epi, st);
+    else return launch_gemm_tc<128, 256>(g, batch, epi, st);
 }
 
 }  // namespace fi
