@@ -245,7 +245,7 @@ struct EpiProj {
 // part are two 16-byte pieces of eight (c, kx) at column (part, y), the MN-major core matrices.  For
 // S <= 128 (both operands and two tiles of v fit an SM: 168 KB at 128); wider grids run the two
 // products of the general kernel.  CH is 8 (all 128 rows of the second product) where that gives
-// enough blocks, else fewer.  32 samples of 128 x 128: 40 us in two kernels -> 28 us (caches
+// enough blocks, else fewer.  32 samples of 128 x 128: 40 us in two kernels -> 26 us (caches
 // flushed); one 64 x 64 sample: inference 170 -> 140 us.
 // ---------------------------------------------------------------------------
 constexpr int DFT2_S = 128;
@@ -254,38 +254,44 @@ struct Dft2Args {
     const bf16 *v, *F1, *F2;
     long long vs;  // sample stride; channels are S*S apart
     bf16* Z;
-    int B, S, CH;
+    int B, CH;
     int* err;
     long long polls;
 };
 inline int dft2_smem(int S) { return DFT2_NB * 256 * S + 64 * S + 512 * S + 256 * S; }
 
+// 16-byte pieces of a K-major operand of n <= R rows (row pitch LD): eight neighbouring threads of the
+// 256 take the rows of one core matrix, the next eight the next eight columns
+template <int R, int LD>
+__device__ __forceinline__ void dft2_stage(uint32_t dst, const bf16* src, int n) {
+    constexpr int KG = LD / 8;
+#pragma unroll
+    for (int v0 = 0; v0 < R * KG; v0 += 256) {
+        const int v = v0 + threadIdx.x, q = v >> 3, rg = q / KG, k = q - rg * KG, r = rg * 8 + (v & 7);
+        if ((R * KG % 256 == 0 || v < R * KG) && r < n)
+            cp_async16(dst + k * (R * 16) + rg * 128 + (v & 7) * 16, src + r * LD + 8 * k, true);
+    }
+}
+
+template <int S>
 __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t tmem_base;
     __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = g.S, CH = g.CH;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, CH = g.CH;
     const int groups = C / CH, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * CH;
-    const int rows = CH * S, nt = (rows + 127) >> 7, kg = S >> 3;
+    const int rows = CH * S, nt = (rows + 127) >> 7;
     const uint32_t sV = tc_smem_u32(smem), sF1 = sV + DFT2_NB * 256 * S, sA = sF1 + 64 * S, sF2 = sA + 512 * S;
-    // 16-byte pieces of a K-major operand of R rows (row pitch ld): eight neighbouring threads take
-    // the rows of one core matrix, the next eight the next eight columns
-    auto stage = [&](uint32_t dst, const bf16* src, int R, int n, int ld, int kgr) {
-        const int total = ((n + 7) >> 3) * 8 * kgr;
-        for (int v = tid; v < total; v += 256) {
-            const int q = v >> 3, rg = q / kgr, k = q - rg * kgr, r = rg * 8 + (v & 7);
-            if (r < n) cp_async16(dst + k * (R * 16) + rg * 128 + (v & 7) * 16, src + (size_t)r * ld + 8 * k, true);
-        }
-    };
-    stage(sF1, g.F1, 32, 32, S, kg);
-    stage(sF2, g.F2, 64, 64, 2 * S, 2 * kg);
+    dft2_stage<32, S>(sF1, g.F1, 32);
+    dft2_stage<64, 2 * S>(sF2, g.F2, 64);
     if (warp == 0) {
         tc_alloc(&tmem_base, 128);
         tc_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&bar, 1);
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
     }
@@ -298,35 +304,51 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
     if (dep_early()) dep_launch();
     // tile t to buffer t % DFT2_NB; a group is committed for every tile, also past the end
     auto stage_tile = [&](int t) {
-        if (t < nt) stage(sV + (t % DFT2_NB) * 256 * S, src + (size_t)t * 128 * S, 128, min(128, rows - t * 128), S, kg);
+        if (t < nt)
+            dft2_stage<128, S>(sV + (t % DFT2_NB) * 256 * S, src + (size_t)t * 128 * S, rows - t * 128);
         cp_async_commit();
     };
     for (int t = 0; t < DFT2_NB - 1; t++) stage_tile(t);
     const int quad = warp & 3, half = warp >> 2, pr = quad * 32 + lane;
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-    int n = 0;  // commits
-    for (int t = 0; t < nt; t++) {
-        stage_tile(t + DFT2_NB - 1);  // its buffer was last read by tile t - 1's product, which is done
-        cp_async_wait<DFT2_NB - 1>();
-        fence_async_smem();
+    // Commit n (tile n; the last one is the second product) goes to bars[n & 1].  A tile's product is
+    // issued before the previous tile's accumulator is read (two accumulators), so it runs beside that
+    // epilogue.
+    int n = 0;
+    auto wait_commit = [&](int c) {
+        if (tid == 0 && !mbar_wait(&bars[c & 1], (uint32_t)((c >> 1) & 1), g.polls)) s_fail = 1;
         __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t a0 = sV + (t % DFT2_NB) * 256 * S;
-            for (int ks = 0; ks < S / 16; ks++)
-                tc_mma(tmem, tc_smem_desc(a0 + 2 * ks * 2048, 2048, 128), tc_smem_desc(sF1 + 2 * ks * 512, 512, 128),
-                       tc_instr_desc(TC_BM, 32), ks > 0);
-            tc_commit(&bar);
-            if (!mbar_wait(&bar, (uint32_t)(n & 1), g.polls)) s_fail = 1;
-        }
-        n++;
-        __syncthreads();
-        if (s_fail) break;
         tc_fence_after();
-        // this thread's row (c, y), part `half`
+        return !s_fail;
+    };
+    bool ok = true;
+    for (int t = 0; t <= nt && ok; t++) {
+        if (t < nt) {
+            cp_async_wait<DFT2_NB - 2>();
+            fence_async_smem();
+            __syncthreads();
+            if (tid == 0) {
+                tc_fence_after();
+                const uint32_t a0 = sV + (t % DFT2_NB) * 256 * S;
+#pragma unroll
+                for (int ks = 0; ks < S / 16; ks++)
+                    tc_mma(tmem + (t & 1) * 32, tc_smem_desc(a0 + 2 * ks * 2048, 2048, 128),
+                           tc_smem_desc(sF1 + 2 * ks * 512, 512, 128), tc_instr_desc(TC_BM, 32), ks > 0);
+                tc_commit(&bars[t & 1]);
+            }
+            n = t + 1;
+        }
+        if (t == 0) {
+            stage_tile(DFT2_NB - 1);
+            continue;
+        }
+        // tile t - 1: this thread's row (c, y), part `half`
+        ok = wait_commit(t - 1);
+        if (!ok) break;
+        if (t < nt) stage_tile(t + DFT2_NB - 1);  // to the buffer of tile t - 1
         float v[16];
-        tc_ld16(tmem + lanes + (uint32_t)(half * 16), v);
-        const int row = t * 128 + pr;
+        tc_ld16(tmem + lanes + (uint32_t)(((t - 1) & 1) * 32 + half * 16), v);
+        const int row = (t - 1) * 128 + pr;
         if (row < rows) {
             const int c = row / S, k = half * S + row - c * S;
             unsigned char* d = smem + (sA - sV) + (k >> 3) * 2048 + (2 * c) * 128 + (k & 7) * 16;
@@ -335,23 +357,22 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
         }
         tc_fence_before();
     }
-    if (!s_fail) {
+    if (ok) {
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
+#pragma unroll
             for (int ks = 0; ks < S / 8; ks++)
                 tc_mma(tD2, tc_smem_desc(sA + 2 * ks * 2048, 2048, 128), tc_smem_desc(sF2 + 2 * ks * 1024, 1024, 128),
                        tc_instr_desc(TC_BM, 64) | (1u << 15), ks > 0);
-            tc_commit(&bar);
-            if (!mbar_wait(&bar, (uint32_t)(n & 1), g.polls)) s_fail = 1;
+            tc_commit(&bars[n & 1]);
         }
         n++;
-        __syncthreads();
+        ok = wait_commit(n - 1);
     }
-    if (!s_fail) {
+    if (ok) {
         if (!dep_early()) dep_launch();
-        tc_fence_after();
         // row m = (c, kx): to shared memory as [kx][kyi][part][c] (the tiles of v are done), then out in
         // runs of CH channels
         bf16* const zt = (bf16*)smem;
@@ -381,7 +402,7 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
     cp_async_wait<0>();
     if (s_fail && tid == 0) {
         if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
-        mbar_wait(&bar, (uint32_t)((n - 1) & 1));  // let the issued MMAs finish before their memory goes
+        mbar_wait(&bars[(n - 1) & 1], (uint32_t)(((n - 1) >> 1) & 1));  // let the issued MMAs finish first
     }
     tc_fence_before();
     __syncthreads();
@@ -1117,14 +1138,18 @@ int finish(fi_fno* h, float* loss = nullptr) {
     return FI_OK;
 }
 
+void (*dft2_kernel(int S))(Dft2Args) {
+    return S == 32 ? k_dft2<32> : S == 64 ? k_dft2<64> : S == 96 ? k_dft2<96> : k_dft2<128>;
+}
+
 // truncated DFT along x and y (F1, F2), or the adjoint of the inverse (G1T, G2T), of 32 channels
 int dft2(fi_fno* h, int B, const bf16* v, long long vs, const bf16* F1, const bf16* F2, bf16* Z) {
     const int S = h->S;
     if (S <= DFT2_S) {
         int CH = 8;
         while (CH > 1 && B * (C / CH) < 96) CH /= 2;
-        const Dft2Args a{v, F1, F2, vs, Z, B, S, CH, h->err, tc_wait_polls()};
-        FNO_CK(launch_dep(k_dft2, B * (C / CH), 256, dft2_smem(S), h->st, a));
+        const Dft2Args a{v, F1, F2, vs, Z, B, CH, h->err, tc_wait_polls()};
+        FNO_CK(launch_dep(dft2_kernel(S), B * (C / CH), 256, dft2_smem(S), h->st, a));
         return FI_OK;
     }
     FNO_CK(gemm(h, C * S, 2 * KX, S, opK(v, S, vs), opK(F1, S), B, EpiDftX{h->Tb, B, S}));
@@ -1251,7 +1276,8 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     if (cudaStreamCreateWithFlags(&h->st, cudaStreamDefault) != cudaSuccess) return bad(FI_ERR_CUDA);
     if (cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaFuncSetAttribute(k_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(k_dft2, cudaFuncAttributeMaxDynamicSharedMemorySize, dft2_smem(DFT2_S)) != cudaSuccess ||
+        (S <= DFT2_S && cudaFuncSetAttribute(dft2_kernel(S), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             dft2_smem(S)) != cudaSuccess) ||
         cudaFuncSetAttribute(k_wgrad<C + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<C + 1>()) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_wgrad<NIN + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<NIN + 1>()) !=
