@@ -116,6 +116,7 @@ struct fi_handle {
     ResArgs rargs{};
     int resident_grid = 0;
     size_t resident_smem = 0;
+    int resident_smem_max = 0;  // the same for every handle, so that threads may set it side by side
     unsigned long long* d_trace = nullptr;  // phase timeline of the persistent executor
     // plain form
     PlainBufs p{};
@@ -1750,6 +1751,7 @@ static int setup_resident(fi_handle* h, int K, int nsm) {
                     h->resident_grid, budget, &r.L))
         return FI_OK;
     h->resident_smem = (size_t)r.L.bytes;
+    h->resident_smem_max = (int)budget;
     h->resident = true;
     return FI_OK;
 }
@@ -1821,7 +1823,7 @@ static int persist_fn(fi_handle* h, const void** out) {
     }
     if (h->resident) {
         const void* r = resident_kernel(sx, sy, h->rargs.L.all);
-        CK(cudaFuncSetAttribute(r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->resident_smem));
+        CK(cudaFuncSetAttribute(r, cudaFuncAttributeMaxDynamicSharedMemorySize, h->resident_smem_max));
         *out = r;
         return FI_OK;
     }

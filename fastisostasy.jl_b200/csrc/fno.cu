@@ -243,111 +243,111 @@ struct EpiProj {
 //   Z[mode][b][part*32 + c] = T[(c, kx)][(part, y)] x F2[(kyi, part')][(part, y)]
 // T exists only as the BF16 operand of the second product in shared memory: a row's 16 values of a
 // part are two 16-byte pieces of eight (c, kx) at column (part, y), the MN-major core matrices.  For
-// S <= 128 (both operands and two tiles of v fit an SM: 168 KB at 128); wider grids run the two
+// S <= 128 (both operands and three tiles of v fit an SM: 201 KB at 128); wider grids run the two
 // products of the general kernel.  CH is 8 (all 128 rows of the second product) where that gives
-// enough blocks, else fewer.  32 samples of 128 x 128: 40 us in two kernels -> 26 us (caches
-// flushed); one 64 x 64 sample: inference 170 -> 140 us.
+// enough blocks, else fewer.  One thread keeps three tiles' TMA loads in flight and issues the MMAs;
+// the other work of a tile is its accumulator's way to shared memory.  With 16-byte cp.async copies
+// by all threads, their issue alone took 2200 cycles of a tile's 4000.
+// 32 samples of 128 x 128: 40 us in two kernels, 26 us fused with cp.async, 14 us
+// (the pass: inference 600 -> 550 us, training step 1483 -> 1386 us).
 // ---------------------------------------------------------------------------
 constexpr int DFT2_S = 128;
-constexpr int DFT2_NB = 3;  // tile buffers: two tiles' copies in flight
+constexpr int DFT2_NB = 3;  // tile buffers
+constexpr int dft2_kb(int S) { return S % 64 ? 32 : 64; }  // columns of a TMA box
 struct Dft2Args {
-    const bf16 *v, *F1, *F2;
-    long long vs;  // sample stride; channels are S*S apart
+    CUtensorMap v, F1, F2;  // v: (x, (c, y), sample), boxes of 128 rows; F1, F2: all rows
     bf16* Z;
     int B, CH;
     int* err;
     long long polls;
 };
-inline int dft2_smem(int S) { return DFT2_NB * 256 * S + 64 * S + 512 * S + 256 * S; }
-
-// 16-byte pieces of a K-major operand of n <= R rows (row pitch LD): eight neighbouring threads of the
-// 256 take the rows of one core matrix, the next eight the next eight columns
-template <int R, int LD>
-__device__ __forceinline__ void dft2_stage(uint32_t dst, const bf16* src, int n) {
-    constexpr int KG = LD / 8;
-#pragma unroll
-    for (int v0 = 0; v0 < R * KG; v0 += 256) {
-        const int v = v0 + threadIdx.x, q = v >> 3, rg = q / KG, k = q - rg * KG, r = rg * 8 + (v & 7);
-        if ((R * KG % 256 == 0 || v < R * KG) && r < n)
-            cp_async16(dst + k * (R * 16) + rg * 128 + (v & 7) * 16, src + r * LD + 8 * k, true);
-    }
-}
+constexpr int dft2_smem(int S) { return DFT2_NB * 256 * S + 64 * S + 256 * S + 512 * S + 1024; }
 
 template <int S>
 __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bars[2];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2], full[DFT2_NB], fbar[2];
     __shared__ uint32_t tmem_base;
-    __shared__ int s_fail;
+    constexpr int KB = dft2_kb(S), BOX = 128 * KB * 2;  // bytes of a box of v
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, CH = g.CH;
     const int groups = C / CH, b = blockIdx.x / groups, c0 = (blockIdx.x - b * groups) * CH;
     const int rows = CH * S, nt = (rows + 127) >> 7;
-    const uint32_t sV = tc_smem_u32(smem), sF1 = sV + DFT2_NB * 256 * S, sA = sF1 + 64 * S, sF2 = sA + 512 * S;
-    dft2_stage<32, S>(sF1, g.F1, 32);
-    dft2_stage<64, 2 * S>(sF2, g.F2, 64);
-    if (warp == 0) {
+    const uint32_t sV = (tc_smem_u32(smem_raw) + 1023) & ~1023u;  // the swizzle's alignment
+    const uint32_t sF1 = sV + DFT2_NB * 256 * S, sF2 = sF1 + 64 * S, sA = sF2 + 256 * S;
+    unsigned char* const smem = smem_raw + (sV - tc_smem_u32(smem_raw));
+    if (tid == 0) {
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&bars[i], 1);
+            mbar_init(&fbar[i], 1);
+        }
+        for (int i = 0; i < DFT2_NB; i++) mbar_init(&full[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+        // the matrices are constants of the network
+        mbar_expect(&fbar[0], 64 * S);
+        for (int x = 0; x < S; x += KB) tma_load(sF1 + x * 64, &g.F1, x, 0, 0, &fbar[0]);
+        mbar_expect(&fbar[1], 256 * S);
+        for (int x = 0; x < 2 * S; x += KB) tma_load(sF2 + x * 128, &g.F2, x, 0, 0, &fbar[1]);
+    }
+    if (warp == 1) {
         tc_alloc(&tmem_base, 128);
         tc_relinquish();
-    }
-    if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_fail = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_base, tD2 = tmem + 64;
-    const bf16* src = g.v + (size_t)b * g.vs + (size_t)c0 * S * S;
+    const uint32_t tmem = tmem_base;  // three accumulators of 32 columns, then the second product's 64
     dep_wait();
     if (dep_early()) dep_launch();
-    // tile t to buffer t % DFT2_NB; a group is committed for every tile, also past the end
-    auto stage_tile = [&](int t) {
-        if (t < nt)
-            dft2_stage<128, S>(sV + (t % DFT2_NB) * 256 * S, src + (size_t)t * 128 * S, rows - t * 128);
-        cp_async_commit();
+    // thread 0: tile t to buffer t % DFT2_NB (the rows of a last, shorter tile are followed by rows of
+    // the next channels, or zeros, which only unread accumulator rows see)
+    auto load_tile = [&](int t) {
+        uint64_t* const bar = &full[t % DFT2_NB];
+        mbar_expect(bar, 256 * S);
+#pragma unroll
+        for (int i = 0; i < S / KB; i++)
+            tma_load(sV + (t % DFT2_NB) * 256 * S + i * BOX, &g.v, i * KB, c0 * S + t * 128, b, bar);
     };
-    for (int t = 0; t < DFT2_NB - 1; t++) stage_tile(t);
+    int nload = 0, nfull = 0, ncommit = 0;  // thread 0: tiles loaded, tiles that arrived, commits
+    if (tid == 0)
+        for (; nload < min(nt, DFT2_NB); nload++) load_tile(nload);
     const int quad = warp & 3, half = warp >> 2, pr = quad * 32 + lane;
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
     // Commit n (tile n; the last one is the second product) goes to bars[n & 1].  A tile's product is
-    // issued before the previous tile's accumulator is read (two accumulators), so it runs beside that
-    // epilogue.
-    int n = 0;
+    // issued before the previous tile's accumulator is read, so it runs beside that epilogue; with three
+    // accumulators the block barrier behind the previous commit's wait is the only one of a tile.
+    bool dead = false;  // thread 0: a wait gave up
     auto wait_commit = [&](int c) {
-        if (tid == 0 && !mbar_wait(&bars[c & 1], (uint32_t)((c >> 1) & 1), g.polls)) s_fail = 1;
-        __syncthreads();
+        if (tid == 0 && !dead) dead = !mbar_wait(&bars[c & 1], (uint32_t)((c >> 1) & 1), g.polls);
+        const int any = __syncthreads_or(dead);
         tc_fence_after();
-        return !s_fail;
+        return !any;
     };
     bool ok = true;
-    for (int t = 0; t <= nt && ok; t++) {
-        if (t < nt) {
-            cp_async_wait<DFT2_NB - 2>();
-            fence_async_smem();
-            __syncthreads();
-            if (tid == 0) {
+    for (int t = 0; t <= nt; t++) {
+        if (t < nt && tid == 0 && !dead) {
+            if (mbar_wait(&full[t % DFT2_NB], (uint32_t)((t / DFT2_NB) & 1), g.polls) &&
+                (t > 0 || mbar_wait(&fbar[0], 0, g.polls))) {
+                nfull = t + 1;
                 tc_fence_after();
                 const uint32_t a0 = sV + (t % DFT2_NB) * 256 * S;
 #pragma unroll
-                for (int ks = 0; ks < S / 16; ks++)
-                    tc_mma(tmem + (t & 1) * 32, tc_smem_desc(a0 + 2 * ks * 2048, 2048, 128),
-                           tc_smem_desc(sF1 + 2 * ks * 512, 512, 128), tc_instr_desc(TC_BM, 32), ks > 0);
+                for (int x = 0; x < S; x += 16)
+                    tc_mma(tmem + (t % 3) * 32, tma_desc<KB>(a0 + x / KB * BOX + x % KB * 2),
+                           tma_desc<KB>(sF1 + x / KB * (64 * KB) + x % KB * 2), tc_instr_desc(TC_BM, 32), x > 0);
                 tc_commit(&bars[t & 1]);
+                ncommit = t + 1;
+            } else {
+                dead = true;
             }
-            n = t + 1;
         }
-        if (t == 0) {
-            stage_tile(DFT2_NB - 1);
-            continue;
-        }
+        if (t == 0) continue;
         // tile t - 1: this thread's row (c, y), part `half`
         ok = wait_commit(t - 1);
         if (!ok) break;
-        if (t < nt) stage_tile(t + DFT2_NB - 1);  // to the buffer of tile t - 1
+        if (tid == 0 && nload < nt) load_tile(nload++);  // to the buffer of tile t - 1
         float v[16];
-        tc_ld16(tmem + lanes + (uint32_t)(((t - 1) & 1) * 32 + half * 16), v);
+        tc_ld16(tmem + lanes + (uint32_t)(((t - 1) % 3) * 32 + half * 16), v);
         const int row = (t - 1) * 128 + pr;
         if (row < rows) {
             const int c = row / S, k = half * S + row - c * S;
@@ -357,19 +357,25 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
         }
         tc_fence_before();
     }
+    const uint32_t tD2 = tmem + 64;  // the third accumulator is done too
     if (ok) {
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
-            tc_fence_after();
+            if (mbar_wait(&fbar[1], 0, g.polls)) {
+                tc_fence_after();
 #pragma unroll
-            for (int ks = 0; ks < S / 8; ks++)
-                tc_mma(tD2, tc_smem_desc(sA + 2 * ks * 2048, 2048, 128), tc_smem_desc(sF2 + 2 * ks * 1024, 1024, 128),
-                       tc_instr_desc(TC_BM, 64) | (1u << 15), ks > 0);
-            tc_commit(&bars[n & 1]);
+                for (int x = 0; x < 2 * S; x += 16)
+                    tc_mma(tD2, tc_smem_desc(sA + x / 8 * 2048, 2048, 128),
+                           tma_desc<KB>(sF2 + x / KB * (128 * KB) + x % KB * 2), tc_instr_desc(TC_BM, 64) | (1u << 15),
+                           x > 0);
+                tc_commit(&bars[nt & 1]);
+                ncommit = nt + 1;
+            } else {
+                dead = true;
+            }
         }
-        n++;
-        ok = wait_commit(n - 1);
+        ok = wait_commit(nt);
     }
     if (ok) {
         if (!dep_early()) dep_launch();
@@ -399,14 +405,16 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
             else *o = *z;
         }
     }
-    cp_async_wait<0>();
-    if (s_fail && tid == 0) {
+    if (dead) {
         if (g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
-        mbar_wait(&bars[(n - 1) & 1], (uint32_t)(((n - 1) >> 1) & 1));  // let the issued MMAs finish first
+        // let the copies and MMAs in flight finish first
+        for (int t = nfull; t < nload; t++) mbar_wait(&full[t % DFT2_NB], (uint32_t)((t / DFT2_NB) & 1));
+        for (int i = 0; i < 2; i++) mbar_wait(&fbar[i], 0);
+        if (ncommit > 0) mbar_wait(&bars[(ncommit - 1) & 1], (uint32_t)(((ncommit - 1) >> 1) & 1));
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, 128);
+    if (warp == 1) tc_dealloc(tmem, 128);
 }
 
 // ---------------------------------------------------------------------------
@@ -968,6 +976,7 @@ struct fi_fno {
          *dz = nullptr, *dYm = nullptr;
     float *zs[NLAYER] = {}, *q = nullptr, *dq = nullptr, *part = nullptr, *scal = nullptr;
     int *map_loc = nullptr, *map_proj = nullptr, *map_lift = nullptr, *err = nullptr;
+    CUtensorMap tm_v[NLAYER], tm_dz, tm_m[4];  // activations and F1, F2, G1T, G2T for k_dft2
     int nsm = 0;
     int fwdB = 0;  // batch of the last forward pass (0: none)
     std::vector<void*> allocs;
@@ -1142,19 +1151,36 @@ void (*dft2_kernel(int S))(Dft2Args) {
     return S == 32 ? k_dft2<32> : S == 64 ? k_dft2<64> : S == 96 ? k_dft2<96> : k_dft2<128>;
 }
 
-// truncated DFT along x and y (F1, F2), or the adjoint of the inverse (G1T, G2T), of 32 channels
-int dft2(fi_fno* h, int B, const bf16* v, long long vs, const bf16* F1, const bf16* F2, bf16* Z) {
+// truncated DFT along x and y (F1, F2), or the adjoint of the inverse (G1T, G2T), of 32 channels; m: the
+// maps of v (dft2_maps)
+int dft2(fi_fno* h, int B, const CUtensorMap& m, bool adjoint, const bf16* v, long long vs, bf16* Z) {
     const int S = h->S;
     if (S <= DFT2_S) {
         int CH = 8;
         while (CH > 1 && B * (C / CH) < 96) CH /= 2;
-        const Dft2Args a{v, F1, F2, vs, Z, B, CH, h->err, tc_wait_polls()};
+        const Dft2Args a{m, h->tm_m[adjoint ? 2 : 0], h->tm_m[adjoint ? 3 : 1], Z, B, CH, h->err, tc_wait_polls()};
         FNO_CK(launch_dep(dft2_kernel(S), B * (C / CH), 256, dft2_smem(S), h->st, a));
         return FI_OK;
     }
-    FNO_CK(gemm(h, C * S, 2 * KX, S, opK(v, S, vs), opK(F1, S), B, EpiDftX{h->Tb, B, S}));
-    FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(F2, 2 * S), 1, EpiModes{Z, B}));
+    const bf16 *M1 = adjoint ? h->G1T : h->F1, *M2 = adjoint ? h->G2T : h->F2;
+    FNO_CK(gemm(h, C * S, 2 * KX, S, opK(v, S, vs), opK(M1, S), B, EpiDftX{h->Tb, B, S}));
+    FNO_CK(gemm(h, KX * B * C, 2 * KY, 2 * S, opK(h->Tb, 2 * S), opK(M2, 2 * S), 1, EpiModes{Z, B}));
     return FI_OK;
+}
+
+// the tensor maps of k_dft2
+bool dft2_maps(fi_fno* h) {
+    const int S = h->S, S2 = h->S2, KB = dft2_kb(S);
+    bool ok = true;
+    for (int l = 0; l < NLAYER; l++)
+        ok = ok && tma_map(&h->tm_v[l], h->vext[l], S, C * S, S, h->maxB, (long long)VC * S2, KB, 128);
+    ok = ok && tma_map(&h->tm_dz, h->dz, S, C * S, S, h->maxB, (long long)C * S2, KB, 128);
+    const bf16* m[4] = {h->F1, h->F2, h->G1T, h->G2T};
+    for (int i = 0; i < 4; i++) {
+        const int K = i % 2 ? 2 * S : S, R = i % 2 ? 2 * KY : 2 * KX;
+        ok = ok && tma_map(&h->tm_m[i], m[i], K, R, K, 1, (long long)R * K, KB, R);
+    }
+    return ok;
 }
 
 int forward(fi_fno* h, int B, const float* x, float* y) {
@@ -1168,7 +1194,7 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
                 EpiLift{h->vext[0], h->params + o.bP, S2}));
     for (int l = 0; l < NLAYER; l++) {
         const float* lp = h->params + o.layer[l];
-        const int rc = dft2(h, B, h->vext[l], vs, h->F1, h->F2, h->Zm[l]);
+        const int rc = dft2(h, B, h->tm_v[l], false, h->vext[l], vs, h->Zm[l]);
         if (rc) return rc;
         // channel mixing, one batch per mode
         FNO_CK(gemm(h, B, 64, 64, opK(h->Zm[l], 64, (long long)B * 64), opK(h->Wm + (size_t)l * NM * 4096, 64, 4096),
@@ -1212,7 +1238,7 @@ int backward(fi_fno* h, int B) {
         int rc = wgrad<C + 1>(h, B, h->vext[l], vs, 32, h->map_loc, o.layer[l]);
         if (rc) return rc;
         // spectral path: adjoint of the inverse DFT along x, then along y
-        rc = dft2(h, B, h->dz, cs, h->G1T, h->G2T, h->dYm);
+        rc = dft2(h, B, h->tm_dz, true, h->dz, cs, h->dYm);
         if (rc) return rc;
         FNO_CK(launch_dep(k_spec_wgrad, NM, 256, 0, h->st, h->Zm[l], h->dYm, gr + o.layer[l], B));
         // adjoint of the channel mixing and of the DFT along y
@@ -1310,7 +1336,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     for (int l = 0; l < NLAYER && ok; l++)
         ok = dalloc(h, &h->zs[l], (size_t)B * C * S2) == cudaSuccess &&
              dalloc(h, &h->Zm[l], (size_t)NM * B * 64) == cudaSuccess;
-    if (!ok) return bad(FI_ERR_CUDA);
+    if (!ok || (S <= DFT2_S && !dft2_maps(h))) return bad(FI_ERR_CUDA);
     // DFT matrices
     std::vector<bf16> mats[8];
     build_dft(S, mats);

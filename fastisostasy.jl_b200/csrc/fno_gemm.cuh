@@ -18,6 +18,7 @@
 // once and how little a tile costs beside its epilogue.  So only the K columns, rows and stages
 // that a product has take copies and shared memory, and blocks walk tiles (launch_gemm_nb).
 #pragma once
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -112,6 +113,48 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t da, uint64_t db
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tc_smem_u32(bar))
                  : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// TMA operands: boxes of `rows` rows x KB elements (KB = 64 or 32: 128- or 64-byte rows) of a K-major
+// BF16 tensor (x, row, depth), one after another in shared memory (1024-byte aligned) with the
+// swizzle of their row size, which is also the operand layout of the descriptor below.
+// ---------------------------------------------------------------------------
+// inner: row length and box columns start at multiples of KB; pitch, dpitch: elements between rows and
+// between depths (multiples of 8).  Rows of a box beyond `rows` are filled with zeros.
+inline bool tma_map(CUtensorMap* m, const void* p, int inner, int rows, long long pitch, int depth, long long dpitch,
+                    int KB, int box_rows) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)depth};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)dpitch * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)KB, (cuuint32_t)box_rows, 1}, one[3] = {1, 1, 1};
+    return ((Encode)f)(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, one,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, KB == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// descriptor of 16 K columns of such a box: 8-row groups 16 KB bytes apart, rows inside them swizzled.
+// The next 16 columns of the box start 32 bytes on.
+template <int KB>
+__device__ __forceinline__ uint64_t tma_desc(uint32_t saddr) {
+    return tc_smem_desc(saddr, 16, 16 * KB) | ((uint64_t)(KB == 64 ? 2 : 4) << 61);
+}
+
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, int x, int row, int depth, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(row), "r"(depth), "r"(tc_smem_u32(bar))
+        : "memory");
 }
 
 // 16 consecutive FP32 columns of this thread's TMEM lane
