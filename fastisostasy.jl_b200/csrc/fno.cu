@@ -9,18 +9,19 @@
 //   y): 512 complex modes, one complex 32 x 32 channel matrix per mode; the inverse is the
 //   real inverse DFT of that truncated half spectrum (weight 1 at kx = 0, 2 otherwise, 1/S^2).
 //
-// Every contraction but the per-mode weight gradient runs on the tcgen05 GEMM of
-// fno_gemm.cuh (BF16 operands, FP32 accumulators in tensor memory):
+// Every contraction but the per-mode weight gradient runs on the tensor cores (tcgen05, BF16
+// operands, FP32 accumulators in tensor memory), on the GEMM of fno_gemm.cuh unless a kernel is named:
 //   DFT along x:   v[(b,c,y)][x]            x F1[(part,kx)][x]            -> T
 //   DFT along y:   T[(kx,b,c)][(part,y)]    x F2[(kyi,part')][(part,y)]   -> Z (per mode)
+//                  (k_dft2: both at once, up to S = 128)
 //   channel mix:   Z[mode][b][(part,ci)]    x Wmat[mode][(part',co)][(part,ci)]  (512 batches)
 //   inverse y:     Y[(b,co,kx)][(kyi,part)] x G2[(y,part')][(kyi,part)]   -> G[(b,y)][co][(kx,part)]
-//   inverse x + pointwise path, one GEMM per row (b, y) of pixels x channels with K = 32 + 32:
+//   inverse x + pointwise path, one product per row (b, y) of pixels x channels with K = 32 + 32 (k_pix):
 //                  [G1[x][(kx,part)] | v[b][ci][y][x]]  x  [G[(b,y)][co][(kx,part)] | Wloc[co][ci]]
 //                  (the activation v read in place from NCHW as an MN-major operand)
-// The backward pass runs the same GEMMs against the transposed matrices, and the weight
-// gradients of the pointwise layers are split-K GEMMs over pixels whose B operand carries a
-// row of ones (bias gradient) and, for the projection, the loss gradient (dQ2).
+// The backward pass runs the same products against the transposed matrices.  The weight gradients of
+// the pointwise layers are split-K products over pixels whose B operand carries a row of ones (bias
+// gradient; k_wgrad) and, for the projection, the loss gradient (dQ2; k_proj_bwd).
 //
 // Activations live in NCHW ([b][c][y*S+x]) only: the pointwise layers and the projection
 // read them as MN-major operands (pixels x channels).  All parameters are FP32 masters
@@ -415,6 +416,133 @@ __global__ void __launch_bounds__(256) k_dft2(const __grid_constant__ Dft2Args g
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tc_dealloc(tmem, 128);
+}
+
+// ---------------------------------------------------------------------------
+// inverse DFT along x + pointwise path of a row of pixels (and the adjoints of both), per row (b, y) and
+// 128 pixels x:
+//   out[x][c] = G1[x][(kx, part)] x G[(b, y)][c][(kx, part)] + v[b][ci][y][x] x W[c][ci]
+// A ring of PIX_NB tiles: thread 256 keeps their TMA loads in flight and issues the MMAs (an accumulator
+// of 32 columns a slot), two groups of four warps take the accumulators in turn.  A slot's barriers: full
+// (its copies arrived), done (its MMAs finished: the accumulator is ready and the copies' place free),
+// taken (the accumulator was read).  What bounds it is the epilogue's traffic (4-byte values of z along
+// the pixels, BF16 activations); as tiles of the general kernel, ten blocks an SM of four warps with
+// cp.async copies, block barriers and copies, products and stores all in phase, 60 us (forward) and
+// 62 us (backward) at 32 samples of 128 x 128, this one 38 and 42 us (bytes: 21 us).
+// ---------------------------------------------------------------------------
+constexpr int PIX_NB = 4, PIX_THREADS = 288, PIX_BLOCKS = 4;  // blocks: an SM (3: training step 1291 us, 4: 1270)
+constexpr int pix_kb(int S) { return S % 64 ? 32 : 64; }      // pixels of a TMA box
+struct PixArgs {
+    CUtensorMap G1, G, v, W;  // (K, x), (K, c, (b, y)), (pixel, ci, b), (ci, c, layer)
+    int S, ntiles, layer;
+    int* err;
+    long long polls;
+};
+inline int pix_smem(int S) { return PIX_NB * (8192 + 2048) + 2048 + (S > 128 ? 2 : 1) * 8192 + 1024; }
+
+template <int KB, class Epi>
+__global__ void __launch_bounds__(PIX_THREADS, PIX_BLOCKS) k_pix(const __grid_constant__ PixArgs g, const Epi epi) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full[PIX_NB], done[PIX_NB], taken[PIX_NB], fbar;
+    __shared__ uint32_t tmem_base;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = g.S;
+    const int mt = (S + 127) >> 7, G1R = min(S, 128);
+    const uint32_t sV = (tc_smem_u32(smem) + 1023) & ~1023u, sG = sV + PIX_NB * 8192, sW = sG + PIX_NB * 2048,
+                   sG1 = sW + 2048;
+    if (tid == 256) {
+        for (int i = 0; i < PIX_NB; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&done[i], 1);
+            mbar_init(&taken[i], 4);
+        }
+        mbar_init(&fbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+        // G1 is a constant of the network
+        mbar_expect(&fbar, mt * G1R * 64 + 2048);
+        for (int m = 0; m < mt; m++) tma_load(sG1 + m * 8192, &g.G1, 0, m * 128, 0, &fbar);
+    }
+    if (warp == 0) {
+        tc_alloc(&tmem_base, 32 * PIX_NB);
+        tc_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    dep_wait();
+    if (dep_early()) dep_launch();
+    const int n = (g.ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // this block's tiles
+    bool dead = false;
+    if (tid == 256) {
+        tma_load(sW, &g.W, 0, 0, g.layer, &fbar);
+        auto load = [&](int i) {
+            const int tile = blockIdx.x + i * gridDim.x, z = tile / mt, m0 = (tile - z * mt) * 128, b = z / S, y = z - b * S;
+            const int q = i % PIX_NB, nbox = min(128, S - m0) / KB;
+            mbar_expect(&full[q], 2048 + nbox * KB * 64);
+            tma_load(sG + q * 2048, &g.G, 0, 0, z, &full[q]);
+            for (int k = 0; k < nbox; k++)
+                tma_load(sV + q * 8192 + k * KB * 64, &g.v, y * S + m0 + k * KB, 0, b, &full[q]);
+        };
+        int nload = 0, nfull = 0, ncommit = 0;
+        for (; nload < min(n, PIX_NB); nload++) load(nload);
+        dead = !mbar_wait(&fbar, 0, g.polls);
+        for (int i = 0; i < n && !dead; i++) {
+            const int q = i % PIX_NB;
+            const uint32_t ph = (uint32_t)(i / PIX_NB) & 1;
+            dead = !mbar_wait(&full[q], ph, g.polls);
+            if (dead) break;
+            nfull = i + 1;
+            dead = i >= PIX_NB && !mbar_wait(&taken[q], ph ^ 1, g.polls);
+            if (dead) break;
+            tc_fence_after();
+            const int m = (int)((blockIdx.x + i * gridDim.x) % mt);
+            const uint32_t d = tmem + 32 * q, id = tc_instr_desc(TC_BM, 32);
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                tc_mma(d, tma_desc<32>(sG1 + m * 8192 + 32 * k), tma_desc<32>(sG + q * 2048 + 32 * k), id, k > 0);
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                tc_mma(d, tma_desc_mn<KB>(sV + q * 8192 + k * KB * 32, KB * 64), tma_desc<32>(sW + 32 * k), id | (1u << 15),
+                       1u);
+            tc_commit(&done[q]);
+            ncommit = i + 1;
+            // the previous tile's slot, when its MMAs are done
+            if (i > 0 && nload < n) {
+                dead = !mbar_wait(&done[(i - 1) % PIX_NB], (uint32_t)((i - 1) / PIX_NB) & 1, g.polls);
+                if (!dead) load(nload++);
+            }
+        }
+        // copies and MMAs in flight finish first (also when it is an epilogue that gave up)
+        mbar_wait(&fbar, 0);
+        for (int i = nfull; i < nload; i++) mbar_wait(&full[i % PIX_NB], (uint32_t)(i / PIX_NB) & 1);
+        if (ncommit > 0) mbar_wait(&done[(ncommit - 1) % PIX_NB], (uint32_t)((ncommit - 1) / PIX_NB) & 1);
+    } else if (warp < 8) {
+        const int quad = warp & 3;
+        for (int i = warp >> 2; i < n; i += 2) {
+            const int tile = blockIdx.x + i * gridDim.x, z = tile / mt, x = (tile - z * mt) * 128 + quad * 32 + lane;
+            const int q = i % PIX_NB;
+            dead = !__all_sync(0xffffffffu, mbar_wait(&done[q], (uint32_t)(i / PIX_NB) & 1, g.polls));
+            if (dead) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = 0; c0 < 32; c0 += 16) {
+                float v[16];
+                tc_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(32 * q + c0), v);
+                if (c0) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&taken[q]);
+                }
+                if (x < S) epi(z, x, c0, v, 16);
+            }
+        }
+    }
+    if (!dep_early()) dep_launch();
+    if (dead && g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc_dealloc(tmem, 32 * PIX_NB);
 }
 
 // ---------------------------------------------------------------------------
@@ -977,6 +1105,7 @@ struct fi_fno {
     float *zs[NLAYER] = {}, *q = nullptr, *dq = nullptr, *part = nullptr, *scal = nullptr;
     int *map_loc = nullptr, *map_proj = nullptr, *map_lift = nullptr, *err = nullptr;
     CUtensorMap tm_v[NLAYER], tm_dz, tm_m[4];  // activations and F1, F2, G1T, G2T for k_dft2
+    CUtensorMap tm_G1, tm_F1T, tm_G, tm_W, tm_WT, tm_pv[NLAYER], tm_pdz;  // for k_pix
     int nsm = 0;
     int fwdB = 0;  // batch of the last forward pass (0: none)
     std::vector<void*> allocs;
@@ -1008,36 +1137,30 @@ cudaError_t dalloc(fi_fno* h, T** p, size_t count) {
 }
 
 // operands: K-major (rows K-contiguous) and MN-major (NCHW read as pixels x channels)
-TcOperand opK(const bf16* p, int ld, long long s = 0, long long s2 = 0) {
+TcOperand opK(const bf16* p, int ld, long long s = 0) {
     TcOperand o;
     o.p = p;
     o.ld = ld;
     o.s = s;
-    o.s2 = s2;
     o.mn = 0;
     return o;
 }
-TcOperand opMN(const bf16* p, int ld, long long s = 0, long long s2 = 0) {
-    TcOperand o = opK(p, ld, s, s2);
+TcOperand opMN(const bf16* p, int ld, long long s = 0) {
+    TcOperand o = opK(p, ld, s);
     o.mn = 1;
     return o;
 }
 
-// C[z] = A[z] B[z]^T over K columns (columns [K1, K) from A2, B2 when K1 > 0); NTHR 128: 128 x 128
-// tiles of 128 threads, 0: the tile and threads that suit N
+// C[z] = A[z] B[z]^T over K columns; NTHR 128: 128 x 128 tiles of 128 threads, 0: the tile and
+// threads that suit N
 template <int NTHR = 0, class Epi>
-cudaError_t gemm(fi_fno* h, int M, int N, int K, TcOperand A, TcOperand B, int batch, const Epi& epi, int zdiv = 1,
-                 TcOperand A2 = TcOperand(), TcOperand B2 = TcOperand(), int K1 = 0) {
+cudaError_t gemm(fi_fno* h, int M, int N, int K, TcOperand A, TcOperand B, int batch, const Epi& epi) {
     TcGemmArgs g;
     g.M = M;
     g.N = N;
     g.K = K;
     g.A = A;
     g.B = B;
-    g.A2 = A2;
-    g.B2 = B2;
-    g.K1 = K1;
-    g.zdiv = zdiv;
     g.err = h->err;
     if constexpr (NTHR == 128) return launch_gemm_tc<128, 128>(g, batch, epi, h->st);
     else return launch_gemm(g, batch, epi, h->st);
@@ -1168,6 +1291,36 @@ int dft2(fi_fno* h, int B, const CUtensorMap& m, bool adjoint, const bf16* v, lo
     return FI_OK;
 }
 
+// inverse DFT along x + pointwise path (m1 = G1, W) or their adjoints (F1T, WlT); v, the activation or
+// gradient, by its map
+template <class Epi>
+int pix(fi_fno* h, int B, const CUtensorMap& m1, const CUtensorMap& v, const CUtensorMap& W, int layer, const Epi& epi) {
+    const int S = h->S, ntiles = B * S * ((S + 127) / 128);
+    const PixArgs a{m1, h->tm_G, v, W, S, ntiles, layer, h->err, tc_wait_polls()};
+    const int grid = std::min(ntiles, PIX_BLOCKS * h->nsm);
+    FNO_CK(launch_dep(pix_kb(S) == 64 ? k_pix<64, Epi> : k_pix<32, Epi>, grid, PIX_THREADS, pix_smem(S), h->st, a, epi));
+    return FI_OK;
+}
+template <class Epi>
+bool pix_attr(int S) {
+    return cudaFuncSetAttribute(pix_kb(S) == 64 ? k_pix<64, Epi> : k_pix<32, Epi>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, pix_smem(256)) == cudaSuccess;
+}
+
+// the tensor maps of k_pix
+bool pix_maps(fi_fno* h) {
+    const int S = h->S, S2 = h->S2, KB = pix_kb(S), G1R = std::min(S, 128);
+    bool ok = tma_map(&h->tm_G1, h->G1, 32, S, 32, 1, 32LL * S, 32, G1R) &&
+              tma_map(&h->tm_F1T, h->F1T, 32, S, 32, 1, 32LL * S, 32, G1R) &&
+              tma_map(&h->tm_G, h->Gt, 32, C, 32, h->maxB * S, 32 * C, 32, C) &&
+              tma_map(&h->tm_W, h->Wl, C, C, C, NLAYER, C * C, 32, C) &&
+              tma_map(&h->tm_WT, h->WlT, C, C, C, NLAYER, C * C, 32, C) &&
+              tma_map(&h->tm_pdz, h->dz, S2, C, S2, h->maxB, (long long)C * S2, KB, C);
+    for (int l = 0; l < NLAYER; l++)
+        ok = ok && tma_map(&h->tm_pv[l], h->vext[l], S2, C, S2, h->maxB, (long long)VC * S2, KB, C);
+    return ok;
+}
+
 // the tensor maps of k_dft2
 bool dft2_maps(fi_fno* h) {
     const int S = h->S, S2 = h->S2, KB = dft2_kb(S);
@@ -1201,10 +1354,10 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
                     NM, EpiMix{h->Yb}));
         // inverse along y: rows (b, c, kx) -> G[(b, y)][c][(kx, part)]
         FNO_CK(gemm(h, B * C * KX, 2 * S, 64, opK(h->Yb, 64), opK(h->G2, 64), 1, EpiIdftY{h->Gt, S}));
-        // inverse along x + pointwise path: batch (b, y), rows x, K = (kx, part) | ci
-        FNO_CK(gemm(h, S, C, 64, opK(h->G1, 2 * KX), opK(h->Gt, 2 * KX, (long long)S * C * 32, (long long)C * 32),
-                    B * S, EpiPixAct{lp + SPEC + C * C, h->zs[l], h->vext[l + 1], S, S2, l < NLAYER - 1 ? 1 : 0}, S,
-                    opMN(h->vext[l], S2, vs, S), opK(h->Wl + (size_t)l * C * C, C), 2 * KX));
+        // inverse along x + pointwise path
+        const int rp = pix(h, B, h->tm_G1, h->tm_pv[l], h->tm_W, l,
+                           EpiPixAct{lp + SPEC + C * C, h->zs[l], h->vext[l + 1], S, S2, l < NLAYER - 1 ? 1 : 0});
+        if (rp) return rp;
     }
     // one thread sums a row's 128 columns in order: 128 threads
     FNO_CK(gemm<128>(h, S2, PW, C, opMN(h->vext[NLAYER], S2, vs), opK(h->Q1b, C), B,
@@ -1245,11 +1398,10 @@ int backward(fi_fno* h, int B) {
         FNO_CK(gemm(h, B, 64, 64, opK(h->dYm, 64, (long long)B * 64), opK(h->WmT + (size_t)l * NM * 4096, 64, 4096),
                     NM, EpiMix{h->Yb}));
         FNO_CK(gemm(h, B * C * KX, 2 * S, 64, opK(h->Yb, 64), opK(h->F2T, 64), 1, EpiIdftY{h->Gt, S}));
-        // adjoint of the DFT along x + the pointwise path: batch (b, y), rows x, K = (kx, part) | co;
-        // then the activation of the layer below (the lift has none)
-        FNO_CK(gemm(h, S, C, 64, opK(h->F1T, 2 * KX), opK(h->Gt, 2 * KX, (long long)S * C * 32, (long long)C * 32),
-                    B * S, EpiPixBwd{l > 0 ? h->zs[l - 1] : nullptr, h->dz, S, S2}, S, opMN(h->dz, S2, cs, S),
-                    opK(h->WlT + (size_t)l * C * C, C), 2 * KX));
+        // adjoint of the DFT along x + the pointwise path; then the activation of the layer below (the
+        // lift has none)
+        rc = pix(h, B, h->tm_F1T, h->tm_pdz, h->tm_WT, l, EpiPixBwd{l > 0 ? h->zs[l - 1] : nullptr, h->dz, S, S2});
+        if (rc) return rc;
     }
     // lift weights and bias: [c][inputs | ones]
     return wgrad<NIN + 1>(h, B, h->xe, (long long)XC * S2, 64, h->map_lift, 0);
@@ -1304,6 +1456,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
         cudaFuncSetAttribute(k_proj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM) != cudaSuccess ||
         (S <= DFT2_S && cudaFuncSetAttribute(dft2_kernel(S), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              dft2_smem(S)) != cudaSuccess) ||
+        !pix_attr<EpiPixAct>(S) || !pix_attr<EpiPixBwd>(S) ||
         cudaFuncSetAttribute(k_wgrad<C + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<C + 1>()) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_wgrad<NIN + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<NIN + 1>()) !=
@@ -1336,7 +1489,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     for (int l = 0; l < NLAYER && ok; l++)
         ok = dalloc(h, &h->zs[l], (size_t)B * C * S2) == cudaSuccess &&
              dalloc(h, &h->Zm[l], (size_t)NM * B * 64) == cudaSuccess;
-    if (!ok || (S <= DFT2_S && !dft2_maps(h))) return bad(FI_ERR_CUDA);
+    if (!ok || !pix_maps(h) || (S <= DFT2_S && !dft2_maps(h))) return bad(FI_ERR_CUDA);
     // DFT matrices
     std::vector<bf16> mats[8];
     build_dft(S, mats);

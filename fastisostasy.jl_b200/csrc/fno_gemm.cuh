@@ -127,15 +127,17 @@ inline bool tma_map(CUtensorMap* m, const void* p, int inner, int rows, long lon
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-        return false;
+    static const Encode f = [] {
+        void* e = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const cudaError_t r = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &e, cudaEnableDefault, &q);
+        return r == cudaSuccess && q == cudaDriverEntryPointSuccess ? (Encode)e : nullptr;
+    }();
+    if (!f) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)depth};
     const cuuint64_t strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)dpitch * 2};
     const cuuint32_t box[3] = {(cuuint32_t)KB, (cuuint32_t)box_rows, 1}, one[3] = {1, 1, 1};
-    return ((Encode)f)(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, one,
+    return f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, one,
                        CU_TENSOR_MAP_INTERLEAVE_NONE, KB == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -147,6 +149,16 @@ __device__ __forceinline__ uint64_t tma_desc(uint32_t saddr) {
     return tc_smem_desc(saddr, 16, 16 * KB) | ((uint64_t)(KB == 64 ? 2 : 4) << 61);
 }
 
+// the same for an MN-major operand: boxes of KB elements along M x 32 K columns, `lbo` bytes apart along
+// M; 16 columns are two groups of 8, 16 KB bytes apart
+template <int KB>
+__device__ __forceinline__ uint64_t tma_desc_mn(uint32_t saddr, uint32_t lbo) {
+    return tc_smem_desc(saddr, lbo, 16 * KB) | ((uint64_t)(KB == 64 ? 2 : 4) << 61);
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc_smem_u32(bar)), "r"(bytes) : "memory");
 }
@@ -205,9 +217,8 @@ inline cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_
 // ---------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------
-// One GEMM operand.  K-major (mn = 0): element (r, k) of batch (z1, z2) at
-// p[z1 * s + z2 * s2 + r * ld + k], rows K-contiguous.  MN-major (mn = 1): at
-// p[z1 * s + z2 * s2 + k * ld + r], each K column contiguous along the rows (an NCHW
+// One GEMM operand.  K-major (mn = 0): element (r, k) of batch z at p[z * s + r * ld + k], rows
+// K-contiguous.  MN-major (mn = 1): at p[z * s + k * ld + r], each K column contiguous along the rows (an NCHW
 // activation read as pixels x channels).  The tensor cores take either form: the shared
 // memory image keeps the same core-matrix grid and only the inside of each 128-byte
 // core matrix is transposed, which bit 15 (A) / 16 (B) of the instruction descriptor
@@ -215,18 +226,14 @@ inline cudaError_t launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_
 struct TcOperand {
     const __nv_bfloat16* p = nullptr;
     int ld = 0;
-    long long s = 0, s2 = 0;
+    long long s = 0;
     int mn = 0;
 };
 
 struct TcGemmArgs {
     int M = 0, N = 0, K = 0;
-    TcOperand A, B;    // product columns [0, K1)
-    TcOperand A2, B2;  // product columns [K1, K) read at column k - K1 (unused when K1 == K)
-    int K1 = 0;        // multiple of 16; 0 means K
+    TcOperand A, B;
     int batch = 1;
-    // two-level batch: with zdiv > 1 batch z is (z / zdiv, z % zdiv), else (z, 0)
-    int zdiv = 1;
     int* err = nullptr;  // set to FI_ERR_TIMEOUT when a wait gives up
     long long polls = TC_SPIN_LIMIT;  // bound of each commit wait (tc_wait_polls())
 };
@@ -248,51 +255,37 @@ __device__ __forceinline__ void cp_async_wait() {
 // kc (<= 64, a multiple of 16) product columns from k0 of one side (A or B) of the product into
 // the canonical layout at shared address dst, zero outside [0, K).  Rows at or beyond nrows are
 // not copied (within a group of 8 rows of an MN-major operand: zero): what the buffer holds there
-// only reaches accumulator rows or columns that no epilogue reads.  Column groups of 8 below K1
-// come from o1, the rest from o2 at column k - K1.  `safe` is any valid global address (the
-// source operand of a zero-filled copy, never read).  do1 / do2: whether o1's / o2's columns are
-// copied (they may still be in place).
+// only reaches accumulator rows or columns that no epilogue reads.  `safe` is any valid global
+// address (the source operand of a zero-filled copy, never read).
 template <int ROWS, int NTHR>
-__device__ __forceinline__ void tc_stage(uint32_t dst, const TcOperand& o1, const TcOperand& o2, bool do1, bool do2,
-                                         int z1, int z2,
-                                         int row0, int nrows, int k0, int kc, int K, int K1, const void* safe) {
+__device__ __forceinline__ void tc_stage(uint32_t dst, const TcOperand& o, int z, int row0, int nrows, int k0, int kc,
+                                         int K, const void* safe) {
     const int left = nrows - row0;
-    // K-major groups: one 16-byte copy = 8 consecutive K elements of one row; a thread keeps its
-    // K group, so its operand and column are fixed.  Eight neighbouring threads take the eight rows
-    // of one core matrix (contiguous in shared memory: no bank conflicts), the next eight the next
-    // K group (contiguous in global memory).
-    if (!(o1.mn && o2.mn)) {
+    if (!o.mn) {
+        // one 16-byte copy = 8 consecutive K elements of one row; a thread keeps its K group.  Eight
+        // neighbouring threads take the eight rows of one core matrix (contiguous in shared memory: no
+        // bank conflicts), the next eight the next K group (contiguous in global memory).
         const int sh = kc <= 16 ? 1 : kc <= 32 ? 2 : 3;
         const int kv = (threadIdx.x >> 3) & ((1 << sh) - 1), gk = k0 + kv * 8;
-        const bool second = gk >= K1;
-        const TcOperand& o = second ? o2 : o1;
-        if (!o.mn && (second ? do2 : do1) && kv * 8 < kc) {
+        if (kv * 8 < kc) {
             const bool kok = gk < K;
             const int r_ = (threadIdx.x >> (3 + sh)) * 8 + (threadIdx.x & 7), step = NTHR >> sh;
             const int rows = left < ROWS ? left : ROWS;
-            const __nv_bfloat16* src = o.p + (size_t)z1 * o.s + (size_t)z2 * o.s2 + (second ? gk - K1 : gk) +
-                                       (size_t)(row0 + r_) * o.ld;
+            const __nv_bfloat16* src = o.p + (size_t)z * o.s + gk + (size_t)(row0 + r_) * o.ld;
             const size_t sstep = (size_t)step * o.ld;
             for (int r = r_; r < rows; r += step, src += sstep)
                 cp_async16(dst + tc_operand_offset(ROWS, r, kv * 8), kok ? (const void*)src : safe, kok);
         }
-    }
-    // MN-major groups: one 16-byte copy = 8 consecutive rows of one K column, stored as
-    // row (k % 8) of core matrix (k / 8, r / 8); eight neighbouring threads take the eight columns of
-    // one core matrix
-    if (o1.mn || o2.mn) {
+    } else {
+        // one 16-byte copy = 8 consecutive rows of one K column, stored as row (k % 8) of core matrix
+        // (k / 8, r / 8); eight neighbouring threads take the eight columns of one core matrix
         constexpr int RV = ROWS / 8;
         for (int v = threadIdx.x; v < RV * kc; v += NTHR) {
             const int rv = (v >> 3) % RV, kc_ = v / (8 * RV) * 8 + (v & 7);
             const int gk = k0 + kc_;
-            const bool second = gk >= K1;
-            const TcOperand& o = second ? o2 : o1;
-            if (!o.mn || !(second ? do2 : do1) || rv * 8 >= left) continue;
-            const int ck = second ? gk - K1 : gk;
+            if (rv * 8 >= left) continue;
             const bool ok = gk < K;
-            const void* src =
-                ok ? (const void*)(o.p + (size_t)z1 * o.s + (size_t)z2 * o.s2 + (size_t)ck * o.ld + row0 + rv * 8)
-                   : safe;
+            const void* src = ok ? (const void*)(o.p + (size_t)z * o.s + (size_t)gk * o.ld + row0 + rv * 8) : safe;
             cp_async16(dst + (kc_ >> 3) * (ROWS * 16) + rv * 128 + (kc_ & 7) * 16, src, ok);
         }
     }
@@ -313,7 +306,6 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nch = NB == 1 ? 1 : (g.K + TC_BK - 1) / TC_BK;
-    const int K1 = g.K1 > 0 ? g.K1 : g.K;
     const int kc0 = g.K < TC_BK ? (g.K + 15) & ~15 : TC_BK;  // columns of a full chunk
     const uint32_t a_bytes = TC_BM * 2 * kc0, stage_bytes = a_bytes + BN * 2 * kc0;
     const uint32_t sbase = tc_smem_u32(smem);
@@ -322,8 +314,7 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
     const unsigned ntiles = mt * nt * (unsigned)g.batch;
     // an operand that is the same for every tile is copied once, where its chunks keep their buffer
     const bool keep = nch <= NB;
-    const bool fixA1 = keep && mt == 1 && g.A.s == 0 && g.A.s2 == 0, fixA2 = keep && mt == 1 && g.A2.s == 0 && g.A2.s2 == 0;
-    const bool fixB1 = keep && nt == 1 && g.B.s == 0 && g.B.s2 == 0, fixB2 = keep && nt == 1 && g.B2.s == 0 && g.B2.s2 == 0;
+    const bool fixA = keep && mt == 1 && g.A.s == 0, fixB = keep && nt == 1 && g.B.s == 0;
     int m0 = 0, n0 = 0, z = 0;  // the tile whose chunks are being copied
     auto stage = [&](unsigned tile, int c, int buf, bool first) {
         if (c == 0) {
@@ -332,13 +323,10 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
             m0 = (int)(mn - nq * mt) * TC_BM;
             n0 = (int)nq * BN;
         }
-        const int z1 = g.zdiv > 1 ? z / g.zdiv : z, z2 = g.zdiv > 1 ? z - z1 * g.zdiv : 0;
         const uint32_t sa = sbase + (uint32_t)buf * stage_bytes;
         const int left = g.K - c * TC_BK, kc = left < kc0 ? (left + 15) & ~15 : kc0;
-        tc_stage<TC_BM, NTHR>(sa, g.A, g.A2, first || !fixA1, first || !fixA2, z1, z2, m0, g.M, c * TC_BK, kc, g.K, K1,
-                              g.A.p);
-        tc_stage<BN, NTHR>(sa + a_bytes, g.B, g.B2, first || !fixB1, first || !fixB2, z1, z2, n0, g.N, c * TC_BK, kc,
-                           g.K, K1, g.A.p);
+        if (first || !fixA) tc_stage<TC_BM, NTHR>(sa, g.A, z, m0, g.M, c * TC_BK, kc, g.K, g.A.p);
+        if (first || !fixB) tc_stage<BN, NTHR>(sa + a_bytes, g.B, z, n0, g.N, c * TC_BK, kc, g.K, g.A.p);
         cp_async_commit();
     };
     unsigned tile = blockIdx.x;
@@ -390,9 +378,8 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
                     // K step ks covers core-matrix columns 2ks and 2ks + 1
                     const uint64_t da = tc_smem_desc(a0 + 2 * ks * (TC_BM * 16), TC_BM * 16, 128);
                     const uint64_t db = tc_smem_desc(b0 + 2 * ks * (BN * 16), BN * 16, 128);
-                    const bool second = c * TC_BK + ks * 16 >= K1;
-                    const uint32_t amn = second ? g.A2.mn : g.A.mn, bmn = second ? g.B2.mn : g.B.mn;
-                    tc_mma(tmem, da, db, idesc | (amn << 15) | (bmn << 16), (c > 0 || ks > 0) ? 1u : 0u);
+                    tc_mma(tmem, da, db, idesc | ((uint32_t)g.A.mn << 15) | ((uint32_t)g.B.mn << 16),
+                           (c > 0 || ks > 0) ? 1u : 0u);
                 }
                 tc_commit(&bars[j & 1]);
                 last_commit = j;
