@@ -552,101 +552,118 @@ constexpr int SLICE = 512;  // pixels per split-K slice (S2 is a multiple of 102
 
 // part[slice][32][NR] = sum over the slice's pixels of dz[32][p] x act[NR][p], one 128 x N tensor-core
 // tile whose rows beyond 32 (and columns beyond NR) hold whatever the operand buffers overlap: only
-// their own, unread, results depend on it.  A slice is one copy of (32 + NR) KB, 32 MMAs and one
-// wait; three blocks an SM keep copies and MMAs of different slices in flight.  As a general
-// product in eight chunks of K, each with a copy, a wait and two block barriers, it took 38 us at
-// 32 samples of 128 x 128 (67 MB read), this one 31 us.
+// their own, unread, results depend on it.  Boxes of 64 pixels come by TMA; a box's MMAs start when it
+// arrives and the next slice's box follows when they are done, so three blocks an SM keep 200 KB of
+// copies in flight; two accumulators leave the first warp a slice's time to store.  Bytes bound it.
+// 32 samples of 128 x 128 (67 MB read): 38 us as a general product in eight chunks of K, 28 us with one
+// cp.async copy of a slice by 256 threads, about 20 us (training step 1237 -> 1196 us).
+struct WgradArgs {
+    CUtensorMap dz, act;  // (pixel, channel, b), boxes of 64 pixels x 32 and NR channels
+    int ns, nslices;
+    float* part;
+    int* err;
+    long long polls;
+};
+constexpr int WG_BOX = 64, WG_NBOX = SLICE / WG_BOX, WG_THREADS = 64, WG_LAG = 2;
 template <int NR>
-__global__ void __launch_bounds__(256) k_wgrad(const bf16* __restrict__ dz, const bf16* __restrict__ act,
-                                               long long act_s, int S2, int nslices, float* part, int* err,
-                                               long long polls) {
-    constexpr int NG = (NR + 7) / 8, N = (NR + 15) / 16 * 16, KG = SLICE / 8;
-    constexpr int A_LBO = 4 * 128, B_LBO = NG * 128, A_BYTES = KG * A_LBO;
+constexpr int wgrad_smem() {  // the last box's 128 rows end 12 KB behind the boxes of dz
+    constexpr int B = WG_NBOX * ((NR + 7) / 8) * 1024;
+    return WG_NBOX * 4096 + (B > 12288 ? B : 12288) + 2048;
+}
+
+template <int NR>
+__global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ WgradArgs g) {
+    constexpr int NG = (NR + 7) / 8, N = (NR + 15) / 16 * 16;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t full[WG_NBOX], done[WG_NBOX], ready[2], taken[2];
     __shared__ uint32_t tmem_base;
-    __shared__ int s_fail;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ns = S2 / SLICE;
-    const uint32_t sa = tc_smem_u32(smem), sb = sa + A_BYTES;
-    // a piece is 8 pixels (16 bytes) of a row r, to row r % 8 of core matrix (pixel group g, r / 8);
-    // eight neighbouring threads take eight rows of one core matrix (contiguous in shared memory),
-    // the next eight the next pixel group (contiguous in global memory)
-    auto stage = [&](int z) {
-        const int b = z / ns;
-        const size_t px = (size_t)(z - b * ns) * SLICE;
-        const bf16* pa = dz + (size_t)b * C * S2 + px;
-        const bf16* pb = act + (size_t)b * act_s + px;
-        for (int v = tid; v < (4 + NG) * 8 * KG; v += 256) {
-            const int rl = v & 7, g = (v >> 3) % KG, rg = v / (8 * KG);
-            if (rg < 4)
-                cp_async16(sa + g * A_LBO + rg * 128 + rl * 16, pa + (size_t)(rg * 8 + rl) * S2 + 8 * g, true);
-            else if ((rg - 4) * 8 + rl < NR)
-                cp_async16(sb + g * B_LBO + (rg - 4) * 128 + rl * 16, pb + (size_t)((rg - 4) * 8 + rl) * S2 + 8 * g,
-                           true);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t sa = (tc_smem_u32(smem) + 1023) & ~1023u, sb = sa + WG_NBOX * 4096;
+    if (tid == 32) {
+        for (int i = 0; i < WG_NBOX; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&done[i], 1);
         }
-        cp_async_commit();
-    };
-    int z = blockIdx.x;
-    if (warp == 0) {
-        tc_alloc(&tmem_base, 64);
-        tc_relinquish();
-    }
-    if (tid == 0) {
-        mbar_init(&bar, 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&ready[i], 1);
+            mbar_init(&taken[i], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_fail = 0;
+        fence_async_smem();
+    }
+    if (warp == 0) {
+        tc_alloc(&tmem_base, 128);
+        tc_relinquish();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     dep_wait();
     if (dep_early()) dep_launch();
-    if (z < nslices) stage(z);
     const uint32_t tmem = tmem_base;
-    int n = 0;  // slices committed
-    for (; z < nslices; z += gridDim.x) {
-        cp_async_wait<0>();
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            for (int ks = 0; ks < SLICE / 16; ks++)
-                tc_mma(tmem, tc_smem_desc(sa + 2 * ks * A_LBO, A_LBO, 128), tc_smem_desc(sb + 2 * ks * B_LBO, B_LBO, 128),
-                       tc_instr_desc(TC_BM, N), ks > 0);
-            tc_commit(&bar);
-            if (!mbar_wait(&bar, (uint32_t)(n & 1), polls)) s_fail = 1;
-        }
-        n++;
-        __syncthreads();
-        if (s_fail) break;
-        tc_fence_after();
-        if (z + (int)gridDim.x < nslices) stage(z + gridDim.x);
-        if (warp == 0) {
-            float* o = part + ((size_t)z * C + lane) * NR;
+    const int n = (g.nslices - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // this block's slices
+    bool dead = false;
+    if (tid == 32) {
+        auto load = [&](int i, int k) {
+            const int z = blockIdx.x + i * gridDim.x, b = z / g.ns, px = (z - b * g.ns) * SLICE + k * WG_BOX;
+            mbar_expect(&full[k], (32 + NR) * 128);
+            tma_load(sa + k * 4096, &g.dz, px, 0, b, &full[k]);
+            tma_load(sb + k * NG * 1024, &g.act, px, 0, b, &full[k]);
+        };
+        // boxes in the order of all slices: loaded, arrived, committed
+        int nload = 0, nfull = 0, ncommit = 0;
+        for (; nload < WG_NBOX; nload++) load(0, nload);
+        for (int i = 0; i < n && !dead; i++) {
+            const uint32_t d = tmem + 64 * (i & 1);
+            if (i >= 2) dead = !mbar_wait(&taken[i & 1], (uint32_t)((i >> 1) - 1) & 1, g.polls);
+            for (int k = 0; k < WG_NBOX && !dead; k++) {
+                dead = !mbar_wait(&full[k], (uint32_t)i & 1, g.polls);
+                if (dead) break;
+                nfull++;
+                tc_fence_after();
 #pragma unroll
-            for (int c0 = 0; c0 < N; c0 += 16) {
-                float v[16];
-                tc_ld16(tmem + c0, v);
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (c0 + i < NR) o[c0 + i] = v[i];
+                for (int x = 0; x < WG_BOX; x += 16)
+                    tc_mma(d, tma_desc<64>(sa + k * 4096 + 2 * x), tma_desc<64>(sb + k * NG * 1024 + 2 * x),
+                           tc_instr_desc(TC_BM, N), k > 0 || x > 0);
+                tc_commit(&done[k]);
+                ncommit++;
+                // the next slice's box to the place of the box WG_LAG before
+                if (ncommit > WG_LAG && nload < n * WG_NBOX) {
+                    const int c = ncommit - 1 - WG_LAG;
+                    dead = !mbar_wait(&done[c % WG_NBOX], (uint32_t)(c / WG_NBOX) & 1, g.polls);
+                    if (!dead) {
+                        load(nload / WG_NBOX, nload % WG_NBOX);
+                        nload++;
+                    }
+                }
             }
-            tc_fence_before();
+            if (!dead) tc_commit(&ready[i & 1]);
         }
-        // the next slice's MMAs are issued after the next __syncthreads()
+        // copies and MMAs in flight finish first
+        for (int c = nfull; c < nload; c++) mbar_wait(&full[c % WG_NBOX], (uint32_t)(c / WG_NBOX) & 1);
+        if (ncommit > 0) mbar_wait(&done[(ncommit - 1) % WG_NBOX], (uint32_t)((ncommit - 1) / WG_NBOX) & 1);
+    } else if (warp == 0) {
+        for (int i = 0; i < n; i++) {
+            dead = !__all_sync(0xffffffffu, mbar_wait(&ready[i & 1], (uint32_t)(i >> 1) & 1, g.polls));
+            if (dead) break;
+            tc_fence_after();
+            float v[N];
+#pragma unroll
+            for (int c0 = 0; c0 < N; c0 += 16) tc_ld16(tmem + 64 * (i & 1) + c0, v + c0);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&taken[i & 1]);
+            float* o = g.part + ((size_t)(blockIdx.x + i * gridDim.x) * C + lane) * NR;
+#pragma unroll
+            for (int c = 0; c < NR; c++) o[c] = v[c];
+        }
     }
     if (!dep_early()) dep_launch();
-    cp_async_wait<0>();
-    if (s_fail && tid == 0) {
-        if (err) atomicExch(err, FI_ERR_TIMEOUT);
-        mbar_wait(&bar, (uint32_t)((n - 1) & 1));  // let the issued MMAs finish before their memory goes
-    }
+    if (dead && g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, 64);
+    if (warp == 0) tc_dealloc(tmem, 128);
 }
-template <int NR>
-constexpr int wgrad_smem() { return SLICE / 8 * (4 + (NR + 7) / 8) * 128 + 1024; }
 
 // ---------------------------------------------------------------------------
 // adjoint of the projection, fused: per slice of SLICE pixels, in tiles of 128 pixels,
@@ -1106,6 +1123,7 @@ struct fi_fno {
     int *map_loc = nullptr, *map_proj = nullptr, *map_lift = nullptr, *err = nullptr;
     CUtensorMap tm_v[NLAYER], tm_dz, tm_m[4];  // activations and F1, F2, G1T, G2T for k_dft2
     CUtensorMap tm_G1, tm_F1T, tm_G, tm_W, tm_WT, tm_pv[NLAYER], tm_pdz;  // for k_pix
+    CUtensorMap tm_wdz, tm_wv[NLAYER], tm_wx;  // for k_wgrad
     int nsm = 0;
     int fwdB = 0;  // batch of the last forward pass (0: none)
     std::vector<void*> allocs;
@@ -1368,19 +1386,29 @@ int forward(fi_fno* h, int B, const float* x, float* y) {
 
 // weight and bias gradients of a pointwise layer: dz x act (NR channels, the last one ones)
 template <int NR>
-int wgrad(fi_fno* h, int B, const bf16* act, long long act_s, int ranges, const int* map, long long base) {
+int wgrad(fi_fno* h, int B, const CUtensorMap& act, int ranges, const int* map, long long base) {
     const int nz = B * h->ns;
-    FNO_CK(launch_dep(k_wgrad<NR>, std::min(nz, 3 * h->nsm), 256, wgrad_smem<NR>(), h->st, h->dz, act, act_s, h->S2, nz,
-                      h->part, h->err, tc_wait_polls()));
+    const WgradArgs a{h->tm_wdz, act, h->ns, nz, h->part, h->err, tc_wait_polls()};
+    FNO_CK(launch_dep(k_wgrad<NR>, std::min(nz, 3 * h->nsm), WG_THREADS, wgrad_smem<NR>(), h->st, a));
     FNO_CK(reduce_map(h->part, h->st, nz, C * NR, ranges, map, h->grads, base));
     return FI_OK;
+}
+
+// the tensor maps of k_wgrad
+bool wgrad_maps(fi_fno* h) {
+    const int S2 = h->S2;
+    bool ok = tma_map(&h->tm_wdz, h->dz, S2, C, S2, h->maxB, (long long)C * S2, WG_BOX, C) &&
+              tma_map(&h->tm_wx, h->xe, S2, XC, S2, h->maxB, (long long)XC * S2, WG_BOX, NIN + 1);
+    for (int l = 0; l < NLAYER; l++)
+        ok = ok && tma_map(&h->tm_wv[l], h->vext[l], S2, VC, S2, h->maxB, (long long)VC * S2, WG_BOX, C + 1);
+    return ok;
 }
 
 // gradients of all parameters from dq (and its BF16 copy) set by k_loss
 int backward(fi_fno* h, int B) {
     const int S = h->S, S2 = h->S2;
     const Offsets& o = h->o;
-    const long long vs = (long long)VC * S2, cs = (long long)C * S2;
+    const long long cs = (long long)C * S2;
     float* gr = h->grads;
     const ProjBwdArgs pb{h->vext[NLAYER], h->Q1b, h->Q1Tb, h->params + o.b1, h->params + o.Q2, h->dq, h->dz, h->part, S2,
                          B * h->ns, h->err, tc_wait_polls()};
@@ -1388,7 +1416,7 @@ int backward(fi_fno* h, int B) {
     FNO_CK(reduce_map(h->part, h->st, B * h->ns, PW * VC, 16, h->map_proj, gr, 0));
     for (int l = NLAYER - 1; l >= 0; l--) {
         // pointwise path weights and bias: [co][ci | ones]
-        int rc = wgrad<C + 1>(h, B, h->vext[l], vs, 32, h->map_loc, o.layer[l]);
+        int rc = wgrad<C + 1>(h, B, h->tm_wv[l], 32, h->map_loc, o.layer[l]);
         if (rc) return rc;
         // spectral path: adjoint of the inverse DFT along x, then along y
         rc = dft2(h, B, h->tm_dz, true, h->dz, cs, h->dYm);
@@ -1404,7 +1432,7 @@ int backward(fi_fno* h, int B) {
         if (rc) return rc;
     }
     // lift weights and bias: [c][inputs | ones]
-    return wgrad<NIN + 1>(h, B, h->xe, (long long)XC * S2, 64, h->map_lift, 0);
+    return wgrad<NIN + 1>(h, B, h->tm_wx, 64, h->map_lift, 0);
 }
 
 int set_loss(fi_fno* h, int B, const float* target, const float* w, const float* dy) {
@@ -1489,7 +1517,7 @@ int fi_fno_create(int32_t S, int32_t max_batch, int32_t device, uint64_t seed, f
     for (int l = 0; l < NLAYER && ok; l++)
         ok = dalloc(h, &h->zs[l], (size_t)B * C * S2) == cudaSuccess &&
              dalloc(h, &h->Zm[l], (size_t)NM * B * 64) == cudaSuccess;
-    if (!ok || !pix_maps(h) || (S <= DFT2_S && !dft2_maps(h))) return bad(FI_ERR_CUDA);
+    if (!ok || !pix_maps(h) || !wgrad_maps(h) || (S <= DFT2_S && !dft2_maps(h))) return bad(FI_ERR_CUDA);
     // DFT matrices
     std::vector<bf16> mats[8];
     build_dft(S, mats);
