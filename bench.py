@@ -120,13 +120,14 @@ def counters(sim):
 
 def launches_between(a, b, executor):
     """Kernels of this library launched between two counter snapshots.  Persistent
-    executor: one k_persist per segment, plus 7 per host-driven right-hand side (the
-    FSAL re-evaluation after an output: gate, 3 convolution, 3 RHS kernels).  Graph and
+    executor: one k_resident (or k_persist) per segment, plus at least 4 per host-driven
+    right-hand side (the FSAL re-evaluation after an output: gate, 3 RHS kernels; the 3
+    convolution kernels of an open gate are not counted).  Graph and
     loop executors: 3 per right-hand side, 3 per sparse update, 1 per segment start."""
     attempts = (b["naccept"] + b["nreject"]) - (a["naccept"] + a["nreject"])
     nf = b["nf"] - a["nf"]
     if executor == 0:
-        return (b["segments"] - a["segments"]) + 7 * max(0, nf - 3 * attempts)
+        return (b["segments"] - a["segments"]) + 4 * max(0, nf - 3 * attempts)
     return 3 * nf + 3 * (b["nsparse"] - a["nsparse"]) + (b["segments"] - a["segments"])
 
 
@@ -197,10 +198,10 @@ def roofline(dev, us_per_bs3, steps_per_launch, executor, grid):
     traffic = None
     tpath = ROOT / "profiles" / "roofline_traffic.json"
     if tpath.exists():
-        per = json.loads(tpath.read_text()).get("k_persist_bytes_per_bs3_step")
+        per = json.loads(tpath.read_text()).get("k_resident_bytes_per_bs3_step")
         if per:
             traffic = round(per * steps_per_launch)
-    return {"bound": "hbm", "kernel": "k_persist" if executor == 0 else "k_rows_fwd/k_cols/k_rows_inv",
+    return {"bound": "hbm", "kernel": "k_resident" if executor == 0 else "k_rows_fwd/k_cols/k_rows_inv",
             "achieved": round(achieved, 1), "peak": peak, "peak_kind": kind, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": traffic,
             "bytes_per_launch": round(per_step * steps_per_launch), "bytes_per_bs3_step": per_step,
@@ -318,7 +319,7 @@ def config5_bench(dev):
             "window": f"{C5_TIMED_YR:g} yr after {C5_WARM_YR:g} yr", "bs3_steps": attempts,
             "us_per_bs3_step": 1e3 * ms / max(1, attempts),
             "rhs_evals_per_s": (c1["nf"] - c0["nf"]) / (ms / 1e3),
-            "roofline": {"bound": "hbm", "kernel": "k_persist", "achieved": round(achieved, 1), "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": "k_resident", "achieved": round(achieved, 1), "peak": peak,
                          "peak_kind": kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
                          "bytes_per_bs3_step": per_step},
             "plain_fp64": {"value": C5_CMP_YR / 1e3 / (plain_ms / 1e3), "unit": "kyr/s",
@@ -745,7 +746,7 @@ def main():
     ap.add_argument("--fno", action="store_true",
                     help="only the surrogate network's training and inference throughput (128^2, batch 32)")
     ap.add_argument("--profile-config5", action="store_true",
-                    help="N=1024: 5 yr warm-up launch, then one 0.2-yr launch of k_persist (ncu capture target)")
+                    help="N=1024: 5 yr warm-up launch, then one 0.2-yr launch of k_resident (ncu capture target)")
     ap.add_argument("--config5", action="store_true",
                     help="only the N=1024 high-resolution case (short window, roofline, rel-L2 vs FP64)")
     ap.add_argument("--config2-full", action="store_true",

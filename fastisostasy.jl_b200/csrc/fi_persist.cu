@@ -19,6 +19,10 @@
 // the four transform plans with their twiddles and the ice-time table are staged in
 // shared memory once per launch.
 //
+// Used where the resident kernel (fi_resident.cuh, the same results bit for bit, 1.3 to 1.6
+// times as fast) does not fit: more row tiles than SMs at an odd height or beyond 16 rows, staged
+// inputs, a forced register build.
+//
 // The grid barrier, the phase timeline marks and the warp-level controller are in
 // fi_grid.cuh.
 #include "fi_grid.cuh"
