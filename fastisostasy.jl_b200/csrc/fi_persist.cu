@@ -54,7 +54,7 @@ __device__ __forceinline__ void persist_body(const PersistArgs& a) {
     // ---- stage the member, the control block, the plans and the ice times ----
     copy_words(&sm, a.mem, sizeof(Member));
     __syncthreads();
-    copy_words(&sc, sm.ctl, sizeof(Ctl));
+    copy_words(&sc, sm.ctl, sizeof(Ctl));  // word by word over the block's threads: used after a barrier
     float2* tw = (float2*)(smem + a.ws_bytes);
     for (int q = 0; q < 4; q++) {
         const FftPlan& p = q == 0 ? sm.px : q == 1 ? sm.py : q == 2 ? sm.pMx : sm.pMy;
@@ -72,6 +72,7 @@ __device__ __forceinline__ void persist_body(const PersistArgs& a) {
         for (int i = tid; i < sm.K; i += RT) st[i] = sm.t_ice[i];
         tice = st;
     }
+    __syncthreads();
     // ---- segment start: loop header of the first attempt ----
     if (tid == 0) {
         Ctl* c = &sc;

@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(res_threads(RES), 1) k_resident(const __grid_c
     // ---- stage the member, the control block, the plans and the ice times ----
     copy_words(&sm, a.mem, sizeof(Member));
     __syncthreads();
-    copy_words(&sc, sm.ctl, sizeof(Ctl));
+    copy_words(&sc, sm.ctl, sizeof(Ctl));  // word by word over the block's threads: used after a barrier
     const Member& m = sm;
     const int nx = m.nx, ny = m.ny, NH = m.NH, h = a.h_rows, sp = m.sp;
     float2* const twx = (float2*)(smem + L.twx);
@@ -379,8 +379,9 @@ __global__ void __launch_bounds__(res_threads(RES), 1) k_resident(const __grid_c
         rc.mnx = fastdiv_magic((unsigned)nx);
         rc.mnh = fastdiv_magic((unsigned)NH);
     }
+    __syncthreads();
     // ---- segment start: loop header of the first attempt ----
-    if (tid == 32) {
+    if (tid == 0) {
         Ctl* c = &sc;
         int active = (c->status == FI_OK) && (c->t < c->t_stop);
         c->pending_output = 0;
