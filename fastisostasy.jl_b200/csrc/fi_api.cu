@@ -116,7 +116,6 @@ struct fi_handle {
     ResArgs rargs{};
     int resident_grid = 0;
     size_t resident_smem = 0;
-    int resident_smem_max = 0;  // the same for every handle, so that threads may set it side by side
     unsigned long long* d_trace = nullptr;  // phase timeline of the persistent executor
     // plain form
     PlainBufs p{};
@@ -448,6 +447,26 @@ static void set_task_counts(fi_handle* h) {
     h->n_crowi = cdiv(h->ny + 2, h->h_conv);
 }
 
+// A kernel's limit of dynamic shared memory is a property of the kernel on the device that every
+// handle, ensemble and thread shares: always all that the device allows beside the kernel's static
+// use, so that none of them lowers another's.
+static cudaError_t smem_open(const void* f, int device, size_t* limit) {
+    int smax = 0;
+    cudaFuncAttributes fa{};
+    cudaError_t e = cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f);
+    if (e != cudaSuccess) return e;
+    *limit = (size_t)smax > fa.sharedSizeBytes ? (size_t)smax - fa.sharedSizeBytes : 0;
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*limit);
+}
+
+static int smem_need(fi_handle* h, const void* f, size_t need) {
+    size_t limit = 0;
+    CK(smem_open(f, h->cfg.device, &limit));
+    if (need > limit) return set_err(h, FI_ERR_CUDA, "shared memory need %zu B exceeds the per-block limit", need);
+    return FI_OK;
+}
+
 static int create_buffers(fi_handle* h) {
     const size_t n = N2(h);
     RET(get_plan(h, h->nx, &h->plan_x));
@@ -550,11 +569,9 @@ static int create_buffers(fi_handle* h) {
                             (const void*)k_conv_rows, (const void*)k_conv_cols, (const void*)k_conv_rows_inv};
         size_t cap = (size_t)smax;
         for (const void* f : fk) {
-            cudaFuncAttributes fa{};
-            CK(cudaFuncGetAttributes(&fa, f));
-            if (fa.sharedSizeBytes >= (size_t)smax) return set_err(h, FI_ERR_CUDA, "static shared memory too large");
-            const size_t dyn = (size_t)smax - fa.sharedSizeBytes;
-            CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            size_t dyn = 0;
+            CK(smem_open(f, h->cfg.device, &dyn));
+            if (dyn == 0) return set_err(h, FI_ERR_CUDA, "static shared memory too large");
             cap = std::min(cap, dyn);
         }
         h->smem_cap = cap;
@@ -576,18 +593,18 @@ static int create_buffers(fi_handle* h) {
         RET(dalloc(h, &p.Ge_hat, M));
         RET(dalloc(h, &p.Gg_hat, M));
         const size_t s1 = fft64_rows_smem(std::max(h->nx, h->Mx), 1), s2 = fft64_cols_smem(std::max(h->ny, h->My), 1);
-        CK(cudaFuncSetAttribute(k_fft64_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
-        CK(cudaFuncSetAttribute(k_fft64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
+        RET(smem_need(h, (const void*)k_fft64_rows, s1));
+        RET(smem_need(h, (const void*)k_fft64_cols, s2));
         const size_t r1 = fft64_rows_smem(h->nx, 1), r2 = fft64_cols_smem(h->ny, 1);
-        CK(cudaFuncSetAttribute(kp_div_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r1));
-        CK(cudaFuncSetAttribute(kp_rows_real, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r1));
-        CK(cudaFuncSetAttribute(kp_spec_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r2));
+        RET(smem_need(h, (const void*)kp_div_rows, r1));
+        RET(smem_need(h, (const void*)kp_rows_real, r1));
+        RET(smem_need(h, (const void*)kp_spec_cols, r2));
     }
     if (h->cfg.form == FI_FORM_FP32) {
         // FP64 transforms of the set-up are needed by both forms
         const size_t s1 = fft64_rows_smem(h->Mx, 1), s2 = fft64_cols_smem(h->My, 1);
-        CK(cudaFuncSetAttribute(k_fft64_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1));
-        CK(cudaFuncSetAttribute(k_fft64_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2));
+        RET(smem_need(h, (const void*)k_fft64_rows, s1));
+        RET(smem_need(h, (const void*)k_fft64_cols, s2));
     }
     CK(cudaStreamSynchronize(h->stream));
     return FI_OK;
@@ -1751,7 +1768,6 @@ static int setup_resident(fi_handle* h, int K, int nsm) {
                     h->resident_grid, budget, &r.L))
         return FI_OK;
     h->resident_smem = (size_t)r.L.bytes;
-    h->resident_smem_max = (int)budget;
     h->resident = true;
     return FI_OK;
 }
@@ -1786,8 +1802,8 @@ static int setup_persist(fi_handle* h, int K) {
     // column tasks outnumber the SMs, else the one sized for a single block (more
     // registers, no spills: with at most one task per SM a second block only adds barrier
     // arrivals); FI_PERSIST_MINB=1|2 forces one
-    CK(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RET(smem_need(h, k2, smem));
+    RET(smem_need(h, k1, smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k2, ROW_THREADS, smem));
     h->persist_minb = (occ >= 2 && std::max(h->n_rows, h->n_cols) > nsm) ? 2 : 1;
     const char* mb = getenv("FI_PERSIST_MINB");
@@ -1823,13 +1839,12 @@ static int persist_fn(fi_handle* h, const void** out) {
     }
     if (h->resident) {
         const void* r = resident_kernel(sx, sy, h->rargs.L.all);
-        CK(cudaFuncSetAttribute(r, cudaFuncAttributeMaxDynamicSharedMemorySize, h->resident_smem_max));
+        RET(smem_need(h, r, h->resident_smem));
         *out = r;
         return FI_OK;
     }
     const void* f = persist_kernel(sx, sy, h->persist_minb);
-    if (f != persist_kernel(0, 0, h->persist_minb))
-        CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->persist_smem));
+    RET(smem_need(h, f, h->persist_smem));
     *out = f;
     return FI_OK;
 }
@@ -2321,7 +2336,8 @@ static bool ensemble_setup_persist(fi_ensemble* e) {
     e->kfn = ens_kernel(!(es && es[0] == '0'));
     if (cudaFuncGetAttributes(&fa, e->kfn) != cudaSuccess) return false;
     if (smem + fa.sharedSizeBytes + 1024 > (size_t)smax) return false;
-    if (cudaFuncSetAttribute(e->kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+    size_t limit = 0;
+    if (smem_open(e->kfn, dev, &limit) != cudaSuccess || smem > limit) return false;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, e->kfn, ROW_THREADS, smem) != cudaSuccess || occ < 1)
         return false;
     const bool okk = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess &&
