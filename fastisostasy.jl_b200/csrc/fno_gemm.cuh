@@ -353,13 +353,17 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
     for (; tile < ntiles; tile += gridDim.x) {
         const int tm0 = m0, tn0 = n0, tz = z;
         const bool more = tile + gridDim.x < ntiles;
+        bool fail = false;  // s_fail as read directly behind its barrier: thread 0 may set it again before the next one
         for (int c = 0; c < nch; c++, j++) {
             if (NB == 2 && (c + 1 < nch || more)) {
                 // the other stage buffer was last read by the MMAs of chunk j - 1
                 if (j >= 1) {
                     if (tid == 0 && !mbar_wait(&bars[(j - 1) & 1], (uint32_t)(((j - 1) >> 1) & 1), g.polls)) s_fail = 1;
                     __syncthreads();
-                    if (s_fail) break;
+                    if (s_fail) {
+                        fail = true;
+                        break;
+                    }
                 }
                 const bool next = c + 1 == nch;
                 stage(next ? tile + gridDim.x : tile, next ? 0 : c + 1, (j + 1) & 1, j + 1 < nch);
@@ -385,7 +389,7 @@ __global__ void __launch_bounds__(NTHR) k_gemm_tc(const __grid_constant__ TcGemm
                 last_commit = j;
             }
         }
-        if (s_fail) break;
+        if (fail) break;
         // tile complete: wait for its MMAs, read the accumulator, hand rows to the epilogue
         if (tid == 0 && !mbar_wait(&bars[(j - 1) & 1], (uint32_t)(((j - 1) >> 1) & 1), g.polls)) s_fail = 1;
         __syncthreads();

@@ -23,3 +23,16 @@ def test_block_copies_are_followed_by_a_barrier(path):
         assert end >= 0, (path.name, c.group(0))
         use = re.search(r"(?<![\w.])" + re.escape(c.group(1)) + r"\b", rest[:end])
         assert not use, f"{path.name}: {c.group(1)} is used before a barrier: {rest[use.start() - 40:use.end() + 40]!r}"
+
+
+@pytest.mark.parametrize("name", ["fno.cu", "fno_gemm.cuh"])
+def test_failure_words_are_read_behind_their_barrier(name):
+    """A block leaves a loop on the shared word that thread 0 sets when a wait gives up: read anywhere
+    but directly behind a block barrier, one warp could see the next wait's answer and leave one barrier
+    before the others."""
+    src = _code(CSRC / name)
+    reads = [m.start() for m in re.finditer(r"if \(s_fail\)", src)]
+    assert reads
+    for i in reads:
+        before = src[:i].rstrip()
+        assert before.endswith("__syncthreads();"), (name, before[-120:])
