@@ -104,7 +104,9 @@ __device__ __forceinline__ void store16(bf16* dst, const float* v) {
 // GEMM epilogues (called per row and 16-column chunk; every N below is a multiple of 16)
 // ---------------------------------------------------------------------------
 
-// 16 consecutive parameters at a multiple of 16 floats (every group's offset is a multiple of 32).  As
+// 16 consecutive parameters at a multiple of 16 floats (every group's offset is a multiple of 32).  The
+// non-coherent loads hold: parameters change in k_adam and in the host's copies alone, and a call ends
+// with a wait for both before another pass starts.  As
 // single loads beside each value's arithmetic they were two of a hidden unit's loads and waits:
 // 32 samples of 128 x 128, inference 482 -> 468 us, training step 1196 -> 1174 us.
 __device__ __forceinline__ void load16(float* d, const float* __restrict__ p) {
@@ -887,7 +889,9 @@ __global__ void __launch_bounds__(256, 2) k_proj_bwd(const __grid_constant__ Pro
 }
 
 // ---------------------------------------------------------------------------
-// element-wise and reduction kernels
+// element-wise and reduction kernels.  Those launched programmatically take plain pointers: what they
+// read may still be written while they wait, which the non-coherent loads of `const __restrict__`
+// parameters do not allow.
 // ---------------------------------------------------------------------------
 
 // x [B][6][S2] FP32 -> NCHW [b][8][S2] BF16 (channel 6 = 1 for the lift's bias gradient)
@@ -916,8 +920,8 @@ __global__ void k_fill_channel(bf16* v, int B, int S2, int ch, float value) {
 // per-sample weights w (1 when null), dq = 2 w (q - t) / n; or a given dy.
 // Writes dq (FP32), its BF16 copy into channel 33 of the last activation buffer, and
 // accumulates sum(dq) (gradient of b2).
-__global__ void __launch_bounds__(256) k_loss(const float* __restrict__ q, const float* __restrict__ target,
-                                              const float* __restrict__ w, const float* __restrict__ dy, int n,
+__global__ void __launch_bounds__(256) k_loss(const float* q, const float* target,
+                                              const float* w, const float* dy, int n,
                                               int S2, float inv_n, float* dq, bf16* vext4, float* part) {
     dep_wait();
     dep_launch();
@@ -958,7 +962,7 @@ __global__ void __launch_bounds__(256) k_loss(const float* __restrict__ q, const
 
 // the per-block partials of k_loss summed in a fixed order (one block): the loss and the
 // output-bias gradient come out the same on every run
-__global__ void __launch_bounds__(256) k_loss_sum(const float* __restrict__ part, int nblk, float* loss, float* gb2) {
+__global__ void __launch_bounds__(256) k_loss_sum(const float* part, int nblk, float* loss, float* gb2) {
     dep_wait();
     dep_launch();
     __shared__ float sl[256], sd[256];
@@ -985,7 +989,7 @@ __global__ void __launch_bounds__(256) k_loss_sum(const float* __restrict__ part
 // spectral weight gradient of one mode (block = mode):
 //   dWr[ci][co] = sum_b dYr[co] Zr[ci] + dYi[co] Zi[ci]
 //   dWi[ci][co] = sum_b dYi[co] Zr[ci] - dYr[co] Zi[ci]
-__global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* __restrict__ Z, const bf16* __restrict__ dY,
+__global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* Z, const bf16* dY,
                                                     float* gW, int B) {
     dep_wait();
     dep_launch();
@@ -1023,8 +1027,8 @@ __global__ void __launch_bounds__(256) k_spec_wgrad(const bf16* __restrict__ Z, 
 // writes every gradient once), in a fixed order, so that gradients are the same on every run:
 // each of at most 64 ranges of `per` consecutive z in order (range y and y + 32 by row y of the
 // block), then the ranges in order.
-__global__ void __launch_bounds__(1024) k_reduce_map(const float* __restrict__ part, int nz, int MN, int per,
-                                                     const int* __restrict__ map, float* grad, long long base) {
+__global__ void __launch_bounds__(1024) k_reduce_map(const float* part, int nz, int MN, int per,
+                                                     const int* map, float* grad, long long base) {
     dep_wait();
     dep_launch();
     __shared__ float sm[64][33];
@@ -1053,7 +1057,7 @@ static cudaError_t reduce_map(const float* part, cudaStream_t st, int nz, int MN
                       base);
 }
 
-__global__ void k_adam(float* p, const float* __restrict__ g, float* m, float* v, long long n, float lr, float b1,
+__global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, float lr, float b1,
                        float b2, float eps, float c1, float c2) {
     dep_wait();
     dep_launch();
@@ -1070,7 +1074,7 @@ __global__ void k_adam(float* p, const float* __restrict__ g, float* m, float* v
 // spectral weights -> real 64 x 64 block matrices [[Wr, -Wi], [Wi, Wr]] (rows part'*32 + co,
 // cols part*32 + ci) and their transposes; grid (mode, layer).  The weights are read and
 // both matrices written along their rows, through a shared-memory copy of the mode.
-__global__ void __launch_bounds__(256) k_pack_spec(const float* __restrict__ params, long long off0, bf16* Wm,
+__global__ void __launch_bounds__(256) k_pack_spec(const float* params, long long off0, bf16* Wm,
                                                    bf16* WmT) {
     dep_wait();
     dep_launch();
@@ -1093,7 +1097,7 @@ __global__ void __launch_bounds__(256) k_pack_spec(const float* __restrict__ par
 }
 
 // pointwise weights -> BF16 operands: P [32][8], Wloc [l][co][ci] and [l][ci][co], Q1 [128][32], [32][128]
-__global__ void k_pack_small(const float* __restrict__ params, Offsets o, bf16* Pb, bf16* Wl, bf16* WlT, bf16* Q1b,
+__global__ void k_pack_small(const float* params, Offsets o, bf16* Pb, bf16* Wl, bf16* WlT, bf16* Q1b,
                              bf16* Q1Tb) {
     dep_wait();
     dep_launch();

@@ -36,3 +36,16 @@ def test_failure_words_are_read_behind_their_barrier(name):
     for i in reads:
         before = src[:i].rstrip()
         assert before.endswith("__syncthreads();"), (name, before[-120:])
+
+
+def test_programmatic_launches_read_coherently():
+    """A kernel launched while the one before it still runs reads what that one writes: its parameters
+    promise nothing that would let the compiler take the non-coherent path, whose data must not change
+    while the kernel lives (the loads would not be ordered behind the wait either)."""
+    src = _code(CSRC / "fno.cu") + _code(CSRC / "fno_gemm.cuh")
+    names = set(re.findall(r"launch_dep\(\(?(k_\w+)", src)) | {"k_pix", "k_dft2"}
+    assert {"k_adam", "k_pack_spec", "k_loss", "k_reduce_map", "k_gemm_tc"} <= names
+    for name in sorted(names):
+        sig = re.search(r"__global__ void[^;{]*?\b" + name + r"\((.*?)\)\s*\{", src, flags=re.S)
+        assert sig, name
+        assert "__restrict__" not in sig.group(1), (name, sig.group(1))
