@@ -558,10 +558,10 @@ __global__ void __launch_bounds__(PIX_THREADS, PIX_BLOCKS) k_pix(const __grid_co
             }
         }
     }
-    if (!dep_early()) dep_launch();
     if (dead && g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
     tc_fence_before();
     __syncthreads();
+    if (!dep_early()) dep_launch();
     if (warp == 0) tc_dealloc(tmem, 32 * PIX_NB);
 }
 
@@ -678,10 +678,10 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(const __grid_constant__ Wg
             for (int c = 0; c < NR; c++) o[c] = v[c];
         }
     }
-    if (!dep_early()) dep_launch();
     if (dead && g.err) atomicExch(g.err, FI_ERR_TIMEOUT);
     tc_fence_before();
     __syncthreads();
+    if (!dep_early()) dep_launch();
     if (warp == 0) tc_dealloc(tmem, 128);
 }
 

@@ -188,7 +188,8 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
 // another kernel touches (it returns when the kernels before have completed and their writes are
 // visible).  It calls dep_launch() after that -- and after it has its tensor memory, which a waiting
 // block of the next kernel must not hold in its place: at once if the grid has at most one block
-// an SM (dep_early), else when its tiles are done.  (Blocks of the next kernel that start early
+// an SM (dep_early) or its blocks have one short piece of work each (the element-wise kernels), else
+// when the block's tiles are done.  One thread's call counts for its block.  (Blocks of the next kernel that start early
 // gather on the SMs that are free first and then walk their equal shares there: 32 samples of
 // 128 x 128, inference 659 us with the late call, 793 with the early one, 695 without.)  What
 // overlaps is the launch latency and the prologue.  One 64 x 64 sample: 228 -> 170 us; training

@@ -49,3 +49,16 @@ def test_programmatic_launches_read_coherently():
         sig = re.search(r"__global__ void[^;{]*?\b" + name + r"\((.*?)\)\s*\{", src, flags=re.S)
         assert sig, name
         assert "__restrict__" not in sig.group(1), (name, sig.group(1))
+
+
+@pytest.mark.parametrize("name", ["k_pix", "k_wgrad"])
+def test_late_launch_waits_for_the_whole_block(name):
+    """One thread's launch_dependents counts for its block: in kernels whose warps have different jobs,
+    some threads none, the late one stands behind the block's last barrier."""
+    src = _code(CSRC / "fno.cu")
+    body = src[re.search(r"__global__ void[^;{]*?\b" + name + r"\(", src).end():]
+    body = body[:body.index("\n}\n")]
+    late = body.index("if (!dep_early()) dep_launch();")
+    assert body.count("dep_launch();") == 2
+    assert body[:late].rstrip().endswith("__syncthreads();")
+    assert "__syncthreads" not in body[late:]
