@@ -46,7 +46,7 @@ struct Plan {
 struct PlainBufs {
     double *u[2], *k14[2], *k2, *k3, *tmp, *uin, *fscratch;
     double *now_u, *ue, *dz, *H, *H_af, *z_b, *z_ss, *s_i, *s_l, *s_m, *s_load, *s_full, *dudt;
-    double *rhs, *bxx, *byy, *bx, *bxy, *Mxx, *Myy, *Mxy, *buf, *cropped, *off, *partial;
+    double *rhs, *Mxx, *Myy, *Mxy, *buf, *cropped, *off, *partial;
     double2 *fftrhs, *P;
     double *D, *eta, *mask, *u_ref, *ue_ref, *z_b_ref, *z_ss_ref, *H_af_ref, *H_tab;
     double *s_sw, *mgr, *moc, *hwater;  // seawater anomaly, masks, water column
@@ -580,7 +580,7 @@ static int create_buffers(fi_handle* h) {
         const size_t M = (size_t)h->Mx * h->My;
         double** bufs[] = {&p.u[0], &p.u[1], &p.k14[0], &p.k14[1], &p.k2, &p.k3, &p.tmp, &p.uin, &p.fscratch,
                            &p.now_u, &p.ue, &p.dz, &p.H, &p.H_af, &p.z_b, &p.z_ss, &p.s_i, &p.s_l, &p.s_m,
-                           &p.s_load, &p.s_full, &p.dudt, &p.rhs, &p.bxx, &p.byy, &p.bx, &p.bxy, &p.Mxx,
+                           &p.s_load, &p.s_full, &p.dudt, &p.rhs, &p.Mxx,
                            &p.Myy, &p.Mxy, &p.buf, &p.D, &p.eta, &p.mask, &p.u_ref, &p.ue_ref, &p.z_b_ref,
                            &p.z_ss_ref, &p.H_af_ref, &p.s_sw, &p.mgr, &p.moc, &p.hwater, &p.tau, &p.u_eq};
         for (double** b : bufs) RET(dalloc(h, b, n));

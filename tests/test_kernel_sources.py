@@ -62,3 +62,18 @@ def test_late_launch_waits_for_the_whole_block(name):
     assert body.count("dep_launch();") == 2
     assert body[:late].rstrip().endswith("__syncthreads();")
     assert "__syncthreads" not in body[late:]
+
+
+def test_plain_form_allocates_what_it_uses():
+    """Every buffer of the plain FP64 form's struct has a use besides its allocation (a plane is 8 bytes
+    a cell in every handle)."""
+    src = _code(CSRC / "fi_api.cu")
+    struct = re.search(r"struct PlainBufs \{(.*?)\n\};", src, flags=re.S)
+    names = re.findall(r"\*\s*(\w+)", struct.group(1))
+    names += re.findall(r", (\w+)(?=[,;\[])", struct.group(1))
+    assert {"fscratch", "rhs", "Mxy"} <= set(names)
+    rest = src[:struct.start()] + src[struct.end():]
+    rest = re.sub(r"double\*\* bufs\[\] = \{.*?\};", "", rest, flags=re.S)
+    rest = re.sub(r"RET\(dalloc\([^;]*;", "", rest)
+    unused = [n for n in names if not re.search(r"\bp\." + n + r"\b", rest)]
+    assert not unused, unused
