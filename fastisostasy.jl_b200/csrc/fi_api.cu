@@ -1736,30 +1736,38 @@ static int plan_layouts(fi_handle* h, int K) {
 
 // Resident kernel: where the row tiles fit one per SM.  Its tile height is the handle's where
 // that gives at most one tile per SM; else the smallest multiple of it that does, if the
-// handle's is even: even heights pair the same rows in the row transforms (with an odd number
-// of rows, if the last tile is one row high as it is with height 2), so the results do not
-// depend on the choice.  Likewise the column tasks take the smallest multiple of the handle's
-// width that leaves one per SM.  FI_PERSIST_RESIDENT=0 keeps k_persist.
+// handle's is even: even heights pair the same rows in the row transforms, so the results do not
+// depend on the choice.  With an odd number of rows the last row is a tile of its own, as with
+// height 2 (another height whose last tile has an odd number of rows pairs other rows there).
+// When the others' height had to leave that one row by itself, 323 rows took 14-row tiles on 24
+// SMs, 351 rows 10-row tiles on 36, and 299, 303 or 599 found none: us per BS3 attempt, then ->
+// now (k_persist), 512 x 351: 131 -> 98 (122), 512 x 323: 168 -> 107 (147), 1024 x 351: 244 -> 150
+// (199), 256 x 303: 192 -> 119 (192).  Over 4- to 14-row tiles, 256 x 300 to 800 x 1600, this kernel
+// takes 0.46 to 0.83 of k_persist's time, so it runs wherever its tiles fit.
+// Likewise the column tasks take the smallest multiple of the handle's width that leaves one per
+// SM.  FI_PERSIST_RESIDENT=0 keeps k_persist.
 static int setup_resident(fi_handle* h, int K, int nsm) {
     h->resident = false;
     const char* e = getenv("FI_PERSIST_RESIDENT");
     if ((e && e[0] == '0') || h->stage_inputs) return FI_OK;
-    int hr = h->h_rows, Br = h->B_cols;
+    int hr = h->h_rows, Br = h->B_cols, tail = 0;
     if (cdiv(h->ny, hr) > nsm) {
-        if (hr % 2) return FI_OK;
-        for (hr += h->h_rows; hr <= 16 && (cdiv(h->ny, hr) > nsm || (h->ny % 2 && h->ny % hr != 1)); hr += h->h_rows) {}
+        tail = h->ny % 2;
+        if (hr % 2 || (tail && h->ny % hr != 1)) return FI_OK;
+        for (hr += h->h_rows; hr <= 16 && cdiv(h->ny - tail, hr) + tail > nsm; hr += h->h_rows) {}
         if (hr > 16 || hr / h->h_rows > RES_MAX_SUB) return FI_OK;
     }
     while (cdiv(h->NH, Br) > nsm && Br + h->B_cols <= 16) Br += h->B_cols;
     ResArgs& r = h->rargs;
     r.p = h->pargs;
     r.p.h_rows = hr;
-    r.p.n_rows = cdiv(h->ny, hr);
+    r.p.n_rows = cdiv(h->ny - tail, hr) + tail;
     r.p.B_cols = Br;
     r.p.n_cols = cdiv(h->NH, Br);
     r.h_sub = h->h_rows;
     r.n_part = h->n_rows;
     r.B_sub = h->B_cols;
+    r.tail = tail;
     h->resident_grid = std::min(nsm, std::max(r.p.n_rows, r.p.n_cols));
     cudaFuncAttributes fa{};
     CK(cudaFuncGetAttributes(&fa, resident_kernel(0, 0, 1)));

@@ -84,7 +84,8 @@ struct ResArgs {
     // the handle's tiles: error-norm partials are kept per h_sub rows (n_part of them) and
     // corner partials per B_sub columns, so that both sums run in the order of the other
     // executors; h_rows and B_cols are multiples of them
-    int h_sub, n_part, B_sub, pad_;
+    int h_sub, n_part, B_sub;
+    int tail;  // 1: the last row is the last tile, whatever the height of the others
 };
 // Fills L for tiles of h rows within `budget` bytes; false when the mandatory buffers do not
 // fit.  grid: blocks of the launch.

@@ -49,10 +49,11 @@ struct RowRanges {
     int y0, y1, loM, hiM, loU, hiU;
 };
 
-__host__ __device__ inline RowRanges row_ranges(int tile, int h, int ny) {
+// the tile of rows [y0, y1) with its halos
+__host__ __device__ inline RowRanges row_ranges_of(int y0, int y1, int ny) {
     RowRanges r;
-    r.y0 = tile * h;
-    r.y1 = r.y0 + h < ny ? r.y0 + h : ny;
+    r.y0 = y0;
+    r.y1 = y1;
     r.loM = (r.y0 == 0) ? 0 : r.y0 - 1;
     r.hiM = (r.y1 == ny) ? ny : r.y1 + 1;
     if (r.y0 == 0) r.hiM = r.hiM > (ny < 3 ? ny : 3) ? r.hiM : (ny < 3 ? ny : 3);
@@ -62,6 +63,9 @@ __host__ __device__ inline RowRanges row_ranges(int tile, int h, int ny) {
     if (r.loM == 0) r.hiU = r.hiU > (ny < 3 ? ny : 3) ? r.hiU : (ny < 3 ? ny : 3);
     if (r.hiM == ny) r.loU = r.loU < ny - 3 ? r.loU : ny - 3;
     return r;
+}
+__host__ __device__ inline RowRanges row_ranges(int tile, int h, int ny) {
+    return row_ranges_of(tile * h, tile * h + h < ny ? tile * h + h : ny, ny);
 }
 
 __host__ __device__ inline int capU_of(int h) { return h + 4 > 5 ? h + 4 : 5; }

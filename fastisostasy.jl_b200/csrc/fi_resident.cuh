@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(res_threads(RES), 1) k_resident(const __grid_c
 
     // ---- this block's row tile ----
     const bool rows_on = bid < a.n_rows;
-    const RowRanges rr = row_ranges(rows_on ? bid : 0, h, ny);
+    const int ty0 = !rows_on ? 0 : ra.tail && bid == a.n_rows - 1 ? ny - 1 : bid * h;
+    const RowRanges rr = row_ranges_of(ty0, ty0 == ny - 1 ? ny : min(ty0 + h, ny - ra.tail), ny);
     const int y0 = rr.y0, y1 = rr.y1, loU = rr.loU, loT = rr.loM;
     const int nU = rr.hiU - loU, n_own = (y1 - y0) * nx, own0 = (y0 - loU) * nx;
     const unsigned int mnx = rc.mnx;
@@ -879,7 +880,7 @@ __global__ void __launch_bounds__(res_threads(RES), 1) k_resident(const __grid_c
                 double s = 0.0;
 #pragma unroll
                 for (int w = 0; w < RT / 32; w++) s += s_red[tid * (RT / 32) + w];
-                m.partial[bid * (h / ra.h_sub) + tid] = s;
+                m.partial[y0 / ra.h_sub + tid] = s;
             }
         }
         grid_arrive(a.bar);

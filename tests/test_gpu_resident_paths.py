@@ -25,9 +25,26 @@ def test_kernel_of_each_size(monkeypatch, nx, ny, grid):
 
 @pytest.mark.parametrize("nx,ny,grid,mask", [
     (350, 350, 117, False), (1024, 1024, 129, False), (1040, 1001, 131, True), (1100, 594, 138, False),
-    (1100, 890, 138, False), (1300, 600, 109, True), (300, 2001, 126, False),
+    (1100, 890, 138, False), (1300, 600, 109, True), (300, 2001, 144, False),
 ])
 def test_large_tiles_bitwise(monkeypatch, nx, ny, grid, mask):
+    a, sa = _run(monkeypatch, True, nx, ny, 3.0, mask)
+    b, sb = _run(monkeypatch, False, nx, ny, 3.0, mask)
+    assert sa["grid"] == grid and sb["grid"] in (SMS, 2 * SMS), (sa["grid"], sb["grid"])
+    assert sa["naccept"] > 2 and sa["nsparse"] >= 1
+    for k in ("naccept", "nreject", "nf", "nsparse"):
+        assert sa[k] == sb[k], (k, sa[k], sb[k])
+    for f in a:
+        assert np.all(np.isfinite(a[f])) and np.array_equal(a[f], b[f]), (f, np.abs(a[f] - b[f]).max())
+
+
+@pytest.mark.parametrize("nx,ny,grid,mask", [
+    (64, 299, 76, False), (64, 303, 77, True), (64, 351, 89, False), (512, 323, 129, False), (96, 645, 109, True),
+    (300, 2003, 144, False), (1040, 1003, 131, True),
+])
+def test_odd_rows_take_their_even_neighbours_height(monkeypatch, nx, ny, grid, mask):
+    """The last of an odd number of rows is a tile of its own; the others are as high as one row fewer
+    asks for (4, 4, 4, 4, 6, 14 and 8 here; the tile before the last row 2, 2, 2, 2, 2, 14 and 2)."""
     a, sa = _run(monkeypatch, True, nx, ny, 3.0, mask)
     b, sb = _run(monkeypatch, False, nx, ny, 3.0, mask)
     assert sa["grid"] == grid and sb["grid"] in (SMS, 2 * SMS), (sa["grid"], sb["grid"])
