@@ -1057,10 +1057,12 @@ static cudaError_t reduce_map(const float* part, cudaStream_t st, int nz, int MN
                       base);
 }
 
+// err: no step from gradients of a pass in which a wait gave up
 __global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, float lr, float b1,
-                       float b2, float eps, float c1, float c2) {
+                       float b2, float eps, float c1, float c2, const int* err) {
     dep_wait();
     dep_launch();
+    if (*err) return;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -1300,13 +1302,20 @@ int pack(fi_fno* h) {
     return FI_OK;
 }
 
-// wait for the stream; read the GEMMs' timeout flag and, if asked, the loss
-int finish(fi_fno* h, float* loss = nullptr) {
+// wait for the stream; read the kernels' timeout flag and, if asked, the loss.  The flag is taken down
+// for the next call; what the failed one wrote is not used: its activations serve no backward pass, and
+// an Adam step (steps: those of the call) was not made.
+int finish(fi_fno* h, float* loss = nullptr, int steps = 0) {
     int e = 0;
     FNO_CK(cudaMemcpyAsync(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->st));
     if (loss) FNO_CK(cudaMemcpyAsync(loss, h->scal, sizeof(float), cudaMemcpyDeviceToHost, h->st));
     FNO_CK(cudaStreamSynchronize(h->st));
-    if (e) return fail(h, e, "a tensor-core GEMM wait gave up");
+    if (e) {
+        h->fwdB = 0;
+        h->adam_t -= steps;
+        FNO_CK(cudaMemsetAsync(h->err, 0, sizeof(int), h->st));
+        return fail(h, e, "a tensor-core GEMM wait gave up");
+    }
     return FI_OK;
 }
 
@@ -1472,7 +1481,7 @@ int adam(fi_fno* h, float lr) {
     const float c1 = (float)(1.0 / (1.0 - std::pow((double)h->beta1, (double)h->adam_t)));
     const float c2 = (float)(1.0 / (1.0 - std::pow((double)h->beta2, (double)h->adam_t)));
     FNO_CK(launch_dep(k_adam, 148 * 8, 256, 0, h->st, h->params, h->grads, h->m, h->v, h->o.total, lr, h->beta1, h->beta2,
-                      h->eps, c1, c2));
+                      h->eps, c1, c2, h->err));
     return pack(h);
 }
 
@@ -1639,7 +1648,7 @@ int fi_fno_train_step_weighted(fi_fno* h, int32_t B, const float* x, const float
     if (!rc) rc = set_loss(h, B, target, w, nullptr);
     if (!rc) rc = backward(h, B);
     if (!rc) rc = adam(h, lr);
-    if (!rc) rc = finish(h, loss);
+    if (!rc) rc = finish(h, loss, 1);
     return rc;
 }
 
@@ -1661,7 +1670,7 @@ int fi_fno_adam(fi_fno* h, float lr) {
     if (!h) return FI_ERR_ARG;
     FNO_CK(cudaSetDevice(h->device));
     int rc = adam(h, lr);
-    return rc ? rc : finish(h);
+    return rc ? rc : finish(h, nullptr, 1);
 }
 
 int fi_fno_set_adam(fi_fno* h, float beta1, float beta2, float eps) {
