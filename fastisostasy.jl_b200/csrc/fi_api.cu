@@ -1356,10 +1356,10 @@ static int conv_plain(fi_handle* h, const double* input, const double2* Ghat, do
     return FI_OK;
 }
 
-// update_diagnostics!(dudt, u, sim, t), one kernel per broadcast of the reference
 static int reduce_host(fi_handle* h, const double* d_partial, int nblk, int stride, double* out);
 
-// The right-hand side at u (stage null), or at a stage vector that u receives.
+// update_diagnostics!(dudt, u, sim, t): the right-hand side at u (stage null), or at a stage vector
+// that u receives.
 static int rhs_plain(fi_handle* h, double t, double* u, double* dudt, const PlainStage* stage) {
     const fi_config& c = h->cfg;
     PlainBufs& p = h->p;
@@ -1761,7 +1761,9 @@ static int plan_layouts(fi_handle* h, int K) {
 // SMs, 351 rows 10-row tiles on 36, and 299, 303 or 599 found none: us per BS3 attempt, then ->
 // now (k_persist), 512 x 351: 131 -> 98 (122), 512 x 323: 168 -> 107 (147), 1024 x 351: 244 -> 150
 // (199), 256 x 303: 192 -> 119 (192).  Over 4- to 14-row tiles, 256 x 300 to 800 x 1600, this kernel
-// takes 0.46 to 0.83 of k_persist's time, so it runs wherever its tiles fit.
+// takes 0.46 to 0.83 of k_persist's time, so it runs wherever its tiles fit.  (Over 140 random sizes
+// and tiles the worst are 0.94 to 0.95 of k_persist's speed, on rows with a prime factor above 100,
+// which spend their time in the generic radix pass.)
 // Likewise the column tasks take the smallest multiple of the handle's width that leaves one per
 // SM.  FI_PERSIST_RESIDENT=0 keeps k_persist.
 static int setup_resident(fi_handle* h, int K, int nsm) {

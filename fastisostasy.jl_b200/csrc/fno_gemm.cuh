@@ -189,11 +189,12 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
 // visible).  It calls dep_launch() after that -- and after it has its tensor memory, which a waiting
 // block of the next kernel must not hold in its place: at once if the grid has at most one block
 // an SM (dep_early) or its blocks have one short piece of work each (the element-wise kernels), else
-// when the block's tiles are done.  One thread's call counts for its block.  (Blocks of the next kernel that start early
-// gather on the SMs that are free first and then walk their equal shares there: 32 samples of
-// 128 x 128, inference 659 us with the late call, 793 with the early one, 695 without.)  What
-// overlaps is the launch latency and the prologue.  One 64 x 64 sample: 228 -> 170 us; training
-// step of 7 samples of 96 x 96: 768 -> 612 us.
+// when the block's tiles are done.  One thread's call counts for its block.  (Blocks of the next
+// kernel that start early gather on the SMs that are free first and then walk their equal shares
+// there: 32 samples of 128 x 128, every product a tile-walking GEMM, inference 659 us with the late
+// call, 793 with the early one, 695 without.  In k_pix and k_wgrad alone it makes no difference:
+// 462 and 466 us, training step 1176 and 1185.)  What overlaps is the launch latency and the
+// prologue.  One 64 x 64 sample: 228 -> 170 us; training step of 7 samples of 96 x 96: 768 -> 612 us.
 // ---------------------------------------------------------------------------
 constexpr unsigned DEP_EARLY_BLOCKS = 148;
 __device__ __forceinline__ bool dep_early() { return gridDim.x <= DEP_EARLY_BLOCKS; }
@@ -255,9 +256,10 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // kc (<= 64, a multiple of 16) product columns from k0 of one side (A or B) of the product into
 // the canonical layout at shared address dst, zero outside [0, K).  Rows at or beyond nrows are
-// not copied (within a group of 8 rows of an MN-major operand: zero): what the buffer holds there
-// only reaches accumulator rows or columns that no epilogue reads.  `safe` is any valid global
-// address (the source operand of a zero-filled copy, never read).
+// not copied: what the buffer holds there only reaches accumulator rows or columns that no epilogue
+// reads.  The rows of an MN-major operand are copied in groups of 8, so their number is a multiple of
+// 8, as every K is (fi_fno_gemm refuses others).  `safe` is any valid global address (the source
+// operand of a zero-filled copy, never read).
 template <int ROWS, int NTHR>
 __device__ __forceinline__ void tc_stage(uint32_t dst, const TcOperand& o, int z, int row0, int nrows, int k0, int kc,
                                          int K, const void* safe) {

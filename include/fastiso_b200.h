@@ -207,7 +207,9 @@ int fi_create(const fi_config* cfg, fi_handle** out);
 int fi_set_field(fi_handle* h, int32_t field, const double* host, size_t n);
 int fi_get_field(fi_handle* h, int32_t field, double* host, size_t n);
 /* The same for callers whose arrays are row-major (element (i,j) at j + i*ny, as numpy's
- * (nx, ny) arrays): the layout changes on the device, in the copy's shadow. */
+ * (nx, ny) arrays).  The layout of u, ue, dudt, dz_ss and the external ice changes on the device,
+ * by a kernel before or after the copy (for up to 8192 cells set by the caller, and for every other
+ * field, on the host). */
 int fi_set_field_rowmajor(fi_handle* h, int32_t field, const double* host, size_t n);
 int fi_get_field_rowmajor(fi_handle* h, int32_t field, double* host, size_t n);
 
